@@ -118,6 +118,9 @@ struct NttJob {
     // public key); group g stores NTT(x) * mul2[0] at dst rows (go * dst_outer + rr) and NTT(x) * mul2[1] per_group rows
     // further on, so dst_outer = 2 * per_group lays the products out as [group][2][per_group][N]
     const u64 *mul2 = nullptr;
+    // Rows the forward transform may keep its values in between its two kernels, one per row of the job, for jobs whose
+    // aux / add rows alias dst; nullptr: the dst rows themselves
+    u64 *mid = nullptr;
     // Inverse epilogue: closing constants per row replaced by fold[rr][4]
     const u64 *fold = nullptr;
 };

@@ -21,6 +21,8 @@ namespace lb {
 constexpr int kKsThreads = 256;
 constexpr int kMaxSteps = 32;
 
+// digits has at least 2 L rows per ciphertext at every level (beta (L + P) >= 2 L) and is free once the inner product
+// has read it, so the closing transforms use it as their rows in between
 struct KsWs {
     u64 *coef, *digits, *cx, *pc, *tmp;
 };
@@ -274,8 +276,9 @@ struct Placement {
     long outer, inner; // row strides between ciphertexts and between the polynomials of one
 };
 
+// mid: batch * ppc * L rows of scratch where add or add1 may alias out (see NttJob::mid)
 static int moddown_into(Context *ctx, int L, int batch, int ppc, const u64 *cx, u64 *pc, u64 *out, Placement po, const u64 *add,
-                        Placement pa, int add_inner, cudaStream_t stream, const u64 *add1 = nullptr, long add1_outer = 0)
+                        Placement pa, int add_inner, u64 *mid, cudaStream_t stream, const u64 *add1 = nullptr, long add1_outer = 0)
 {
     const HostParams &hp = ctx->hp;
     const int P = hp.size_P, LP = L + P;
@@ -316,6 +319,7 @@ static int moddown_into(Context *ctx, int L, int batch, int ppc, const u64 *cx, 
     fwd.add_inner = add ? add_inner : 0;
     fwd.add1 = add1;
     fwd.add1_outer = add1_outer;
+    fwd.mid = mid;
     return ntt_forward(ctx, fwd, stream);
 }
 
@@ -356,7 +360,7 @@ int moddown(Context *ctx, int L, const u64 *cx, u64 *out, cudaStream_t stream)
     if (rc) return rc;
     KsWs w;
     if ((rc = get_ws(ctx, L, 1, w))) return rc;
-    return moddown_into(ctx, L, 1, 1, cx, w.pc, out, Placement{L, L}, nullptr, Placement{0, 0}, 0, stream);
+    return moddown_into(ctx, L, 1, 1, cx, w.pc, out, Placement{L, L}, nullptr, Placement{0, 0}, 0, nullptr, stream);
 }
 
 // out(b, p) = (p < add_inner ? add(b, p) : 0) + moddown(<modup(cks_b), evk>)_p for a batch of ciphertexts
@@ -378,7 +382,7 @@ static int keyswitch_batch(Context *ctx, int L, int batch, const u64 *cks, long 
         if ((rc = inner_product_steps(ctx, L, nb, w.digits, cks_b, cks_stride, args, w.cx, stream))) return rc;
         const u64 *add_b = add ? add + ((size_t)b0 * pa.outer << hp.logN) : nullptr;
         u64 *out_b = out + ((size_t)b0 * po.outer << hp.logN);
-        if ((rc = moddown_into(ctx, L, nb, 2, w.cx, w.pc, out_b, po, add_b, pa, add_inner, stream))) return rc;
+        if ((rc = moddown_into(ctx, L, nb, 2, w.cx, w.pc, out_b, po, add_b, pa, add_inner, w.digits, stream))) return rc;
     }
     return LB_OK;
 }
@@ -469,7 +473,7 @@ int rotate(Context *ctx, int L, int batch, u64 *ct, int elt_idx, const u64 *glk,
         args.evk[0] = glk;
         args.n_steps = 1;
         if ((rc = inner_product_steps(ctx, L, nb, w.digits, w.tmp + poly, 2L * L, args, w.cx, stream))) return rc;
-        if ((rc = moddown_into(ctx, L, nb, 2, w.cx, w.pc, ct_b, p2, w.tmp, p2, 1, stream, accumulate ? ct_b + poly : nullptr, 2L * L)))
+        if ((rc = moddown_into(ctx, L, nb, 2, w.cx, w.pc, ct_b, p2, w.tmp, p2, 1, w.digits, stream, accumulate ? ct_b + poly : nullptr, 2L * L)))
             return rc;
     }
     return LB_OK;
@@ -524,7 +528,7 @@ int hoisting(Context *ctx, int L, int batch, u64 *ct, int n_steps, const int *el
         count_launch("galois_sum_kernel", stream);
         galois_sum_kernel<<<(int)blocks, kKsThreads, 0, stream>>>(ct_b, 2L * L, w.tmp, ctx->d_mc, args, hp.logN, L, total, accumulate ? 1 : 0);
         LB_CUDA(cudaGetLastError());
-        if ((rc = moddown_into(ctx, L, nb, 2, w.cx, w.pc, ct_b, Placement{2L * L, L}, w.tmp, Placement{L, L}, 1, stream,
+        if ((rc = moddown_into(ctx, L, nb, 2, w.cx, w.pc, ct_b, Placement{2L * L, L}, w.tmp, Placement{L, L}, 1, w.digits, stream,
                                accumulate ? ct_b + poly : nullptr, 2L * L)))
             return rc;
     }

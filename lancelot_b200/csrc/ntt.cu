@@ -8,26 +8,22 @@
 //   inverse: the exact inverse map (the reference halves in every butterfly; here N^-1 is
 //            folded into the last stage).
 //
-// Schedule (new): ONE kernel per transform and one pass over HBM.  A limb of N = 2^16
-// coefficients (512 KiB) does not fit one SM, so a thread-block cluster of C = N / 8192 CTAs
-// owns a limb.  The first log2(C) stages run in registers on coalesced strided global loads;
-// their outputs are scattered to the owning CTA through distributed shared memory; each
-// CTA then finishes an independent 8192-point transform in its own shared memory with
-// register-blocked radix-8 passes and writes its contiguous part of the result with
-// 16-byte stores.  The inverse mirrors this (contiguous loads, local passes, DSMEM gather,
-// last log2(C) stages in registers, coalesced strided stores).  Algorithmic traffic is
-// 16 bytes per coefficient per transform; twiddles (16 B each, value + Shoup quotient) are
-// read through L2.
+// Schedules: rings of 4096 to 65536 points take the two-kernel transforms of ntt_twopass.cuh.  The kernels in this
+// file serve the rest: rings below 4096 points (one block holds a limb in shared memory) and 131072 points, where a
+// thread-block cluster of 16 blocks owns a limb: the first log2(C) stages run in registers on coalesced strided global
+// loads, their outputs are scattered to the owning block through distributed shared memory, and each block finishes
+// an independent 8192-point transform in its own shared memory with register-blocked radix-8 passes.  The inverse
+// mirrors this.
 #include <cooperative_groups.h>
 
 #include "context.h"
-#include "ntt_butterfly.cuh"
+#include "ntt_stages.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace lb {
 
-// Launch shape: threads per CTA, CTAs per SM the register allocation aims at, and log2 of the points one
+// Launch shape of the single-kernel transforms: threads per CTA, CTAs per SM the register allocation aims at, and log2 of the points one
 // CTA keeps in shared memory (8192 points: 64 KiB + padding, three CTAs per SM).  Register passes take at most
 // three stages (radix 8).
 constexpr int kNttThreads = 256;
@@ -51,6 +47,8 @@ struct NttK {
     const u64 *add1; // addend rows of the groups with inner == 1, if they sit elsewhere (see NttJob::add1)
     long add1_outer;
     const u64 *mul2; // forward epilogue: two products per row (see NttJob::mul2)
+    int n_polys, poly_step, log_polys; // row kernels: how polynomials of one prime share a block (see row_place)
+    u64 *mid;        // two-kernel forward transform: rows between the kernels, or nullptr: the dst rows
     const u64 *presub, *presub_scal, *presub_scal_s;
     const signed char *esmall;
     const signed char *small;
@@ -636,362 +634,11 @@ __global__ void __launch_bounds__(kNttThreads, kNttMinBlocks) ntt_inv_kernel(con
     }
 }
 
-// ---- fixed schedule for rings of 8192 points and more ---------------------------------------------
-// Every production ring degree leaves 8192 points per CTA, so the local transform is always the
-// same thirteen stages.  With the stage numbers known at compile time the index arithmetic of a
-// register group collapses to one shared-memory address plus immediate offsets, and the split
-//   first pass : log2(C) + 1 stages on strided global loads (the cluster stages and the first
-//                local one), scattered through distributed shared memory,
-//   pass A     : local stages with spans 2048, 1024, 512 (CTA-wide),
-//   passes B-D : spans 256..1 inside each warp's 1024-point chunk (warp barriers only),
-// makes every register pass a radix-8 one: five passes instead of six.  The inverse mirrors it.
-constexpr int kHalfLoc = 4096;                                // points per half of a CTA's part
-constexpr int kHalfLocPad = kHalfLoc + (kHalfLoc >> 4);        // the same distance in padded shared memory
+} // namespace lb
 
-// offset of element i of a register group in padded shared memory; the group's elements are
-// 2^LOGST apart and its base has zero bits where the element index goes
-template <int LOGST>
-LB_D constexpr int pad_off(const int i)
-{
-    return LOGST >= 4 ? (i << LOGST) + (i << (LOGST - 4)) : LOGST == 3 ? 8 * i + (i >> 1) : i;
-}
+#include "ntt_twopass.cuh"
 
-LB_D uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-LB_D uint32_t map_to_cta(const uint32_t addr, const unsigned rank)
-{
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-LB_D void st_cluster(const uint32_t addr, const u64 v) { asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory"); }
-LB_D u64 ld_cluster(const uint32_t addr)
-{
-    u64 v;
-    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(addr) : "memory");
-    return v;
-}
-
-// group index of iteration `it` (0..3): shared out over the CTA, or inside the warp's own chunk
-template <bool WIDE>
-LB_D int fixed_group(const int it)
-{
-    return WIDE ? (int)threadIdx.x + 256 * it : (int)((threadIdx.x >> 5) << 7) + (int)(threadIdx.x & 31) + 32 * it;
-}
-
-// PLAIN: the input is the limb itself and the output is stored as it is, so none of the fused
-// conversions is compiled in (sixteen inlined copies of the input ones make the instruction stream
-// of this pass miss the cache).
-template <int LOGC, int MODE, bool PLAIN>
-LB_D void fwd_first_fixed(u64 *sm, const FwdIn &in, const unsigned c, const ulonglong2 *tw, const u64 bq, const u64 bq2)
-{
-    constexpr int F = LOGC + 1, R0 = 1 << F, COLS = kHalfLoc >> LOGC;
-    const uint32_t sbase = smem_addr(sm);
-    const u64 q = in.q; // the prime as an integer for the loaders; bq, bq2 are the butterflies' scalars
-    for (int col = threadIdx.x; col < COLS; col += 256) {
-        const int j = c * COLS + col;
-        u64 v[R0];
-        if (PLAIN) {
-#pragma unroll
-            for (int k = 0; k < R0; ++k) v[k] = in.src[j + k * kHalfLoc];
-        } else if (in.small) {
-            // the small polynomial of an encryption as signed bytes, the same for every prime
-            int ev[R0];
-#pragma unroll
-            for (int k = 0; k < R0; ++k) ev[k] = in.small[j + k * kHalfLoc];
-#pragma unroll
-            for (int k = 0; k < R0; ++k) v[k] = ev[k] < 0 ? q - (u64)(-ev[k]) : (u64)ev[k];
-        } else if (in.n == 0 && in.sub == nullptr) {
-            // a plain row in the instantiation with fused parts (its epilogue is what this launch is after)
-#pragma unroll
-            for (int k = 0; k < R0; ++k) v[k] = in.src[j + k * kHalfLoc];
-        } else if (in.n == 1 && in.mat == nullptr) {
-            // One source row reduced into this prime (every conversion of a chain with one special
-            // prime).  The branches on the optional parts stay outside the loops so that all loads
-            // of a part are in flight together; inside load_in each element would wait for its own.
-#pragma unroll
-            for (int k = 0; k < R0; ++k) v[k] = in.src[j + k * kHalfLoc];
-            if (in.es) {
-                int ev[R0];
-#pragma unroll
-                for (int k = 0; k < R0; ++k) ev[k] = in.es[j + k * kHalfLoc];
-#pragma unroll
-                for (int k = 0; k < R0; ++k) {
-                    const u64 x = add_mod(v[k], ev[k] < 0 ? in.es_p - (u64)(-ev[k]) : (u64)ev[k], in.es_p);
-                    v[k] = sub_mod(barrett64(x, q, in.r1), ev[k] < 0 ? q - (u64)(-ev[k]) : (u64)ev[k], q);
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < R0; ++k) v[k] = barrett64(v[k], q, in.r1);
-            }
-            if (in.sub) {
-#pragma unroll
-                for (int h = 0; h < R0; h += 8) {
-                    u64 t[R0 < 8 ? R0 : 8];
-#pragma unroll
-                    for (int k = 0; k < (R0 < 8 ? R0 : 8); ++k) t[k] = in.sub[j + (h + k) * kHalfLoc];
-#pragma unroll
-                    for (int k = 0; k < (R0 < 8 ? R0 : 8); ++k) v[h + k] = sub_mod(v[h + k], shoup_mul(t[k], in.sub_w, in.sub_ws, q), q);
-                }
-            }
-        } else if (in.mat != nullptr && in.sub == nullptr) {
-            // base conversion of several source rows: four outputs share one walk over the rows, so four
-            // loads are in flight per row instead of one
-            constexpr int G = R0 < 4 ? R0 : 4;
-#pragma unroll
-            for (int h = 0; h < R0; h += G) {
-                u128d acc[G];
-#pragma unroll
-                for (int k = 0; k < G; ++k) acc[k] = u128d{0, 0};
-                for (int i = 0; i < in.n; ++i) {
-                    const u64 m = __ldg(in.mat + i);
-                    const u64 *row = in.src + ((size_t)i << in.logN) + j;
-#pragma unroll
-                    for (int k = 0; k < G; ++k) mac_wide(acc[k], row[(h + k) * kHalfLoc], m);
-                }
-#pragma unroll
-                for (int k = 0; k < G; ++k) v[h + k] = barrett128(acc[k], q, in.r0, in.r1);
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < R0; ++k) v[k] = load_in(in, j + k * kHalfLoc);
-        }
-        if (is_f64_mode(MODE)) {
-#pragma unroll
-            for (int k = 0; k < R0; ++k) v[k] = bits_of(f64_from_u52(v[k]));
-        }
-        if (MODE == kF64Tight) {
-#pragma unroll
-            for (int k = 0; k < R0; ++k) v[k] = bits_of(f64_centre(f64_of(v[k]), f64_of(bq), f64_of(bq2)));
-        }
-        fwd_core<F, MODE>(v, tw, 1u, bq, bq2);
-        const int s0 = sidx(j);
-        if constexpr (LOGC == 0) {
-            sm[s0] = v[0];
-            sm[s0 + kHalfLocPad] = v[1];
-        } else {
-            // every CTA of the cluster must be running before its shared memory is written
-            if (col == (int)threadIdx.x) cg::this_cluster().barrier_wait();
-#pragma unroll
-            for (int r = 0; r < (1 << LOGC); ++r) {
-                const uint32_t ra = map_to_cta(sbase + 8u * s0, r);
-                st_cluster(ra, v[2 * r]);
-                st_cluster(ra + 8u * kHalfLocPad, v[2 * r + 1]);
-            }
-        }
-    }
-}
-
-// three forward stages starting at span 2^LOGT
-// q, q2: the butterflies' scalars; qi, r1: the prime as an integer and floor(2^64 / q) for the closing pass
-template <int LOGT, int MODE, bool PLAIN = false>
-LB_D void fwd_pass_fixed(u64 *sm, u64 *gdst, const unsigned cc, const ulonglong2 *tw, const u64 q, const u64 q2, const u64 qi,
-                         const u64 r1, const FwdEpi &epi)
-{
-    constexpr int LOGST = LOGT - 2;
-    constexpr bool WIDE = LOGT + 1 > 10, CLOSING = LOGST == 0;
-    for (int it = 0; it < 4; ++it) {
-        const int g = fixed_group<WIDE>(it);
-        const int lo = g & ((1 << LOGST) - 1), hi = g >> LOGST;
-        const int base = (hi << (LOGT + 1)) + lo;
-        u64 *p = sm + sidx(base);
-        u64 v[8];
-        u64 t[8];
-        if (CLOSING && !PLAIN && epi.aux) load_contig<8>(t, epi.aux + base); // in flight during the butterflies
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = p[pad_off<LOGST>(i)];
-        if (MODE == kF64Tight) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = bits_of(f64_centre(f64_of(v[i]), f64_of(q), f64_of(q2)));
-        }
-        fwd_core<3, MODE>(v, tw, (cc << (12 - LOGT)) + hi, q, q2);
-        if constexpr (CLOSING) {
-            if (is_f64_mode(MODE)) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = f64_canon(f64_of(v[i]), f64_of(q), f64_of(q2));
-            } else if (MODE == kIntLazy) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = barrett64(v[i], qi, r1);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = csub(csub(csub(v[i], q2 << 1), q2), q);
-            }
-            if (!PLAIN && epi.aux) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = shoup_mul(sub_mod(t[i], v[i], qi), epi.scal, epi.scal_s, qi);
-                if (epi.add) {
-                    load_contig<8>(t, epi.add + base);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) v[i] = add_mod(v[i], t[i], qi);
-                }
-            }
-            if (!PLAIN && epi.mul0) {
-                u64 w[8];
-                load_contig<8>(t, epi.mul1 + base);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) w[i] = mul_mod(v[i], t[i], qi, epi.r0, epi.r1);
-                store_contig<8>(w, gdst + epi.dst1_off + base);
-                load_contig<8>(t, epi.mul0 + base);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = mul_mod(v[i], t[i], qi, epi.r0, epi.r1);
-            }
-            store_contig<8>(v, gdst + base);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) p[pad_off<LOGST>(i)] = v[i];
-        }
-    }
-}
-
-template <int LOGC, int MODE, bool PLAIN>
-LB_D void fwd_body_fixed(u64 *sm, const FwdRow &fr, const unsigned c)
-{
-    const u64 q = bf_scalar_q<MODE>(fr.q), q2 = bf_scalar_q2<MODE>(fr.q);
-    const unsigned cc = (1u << LOGC) + c;
-    fwd_first_fixed<LOGC, MODE, PLAIN>(sm, fr.in, c, fr.tw, q, q2);
-    if constexpr (LOGC > 0) cg::this_cluster().sync(); // all scatters into this CTA have landed
-    else __syncthreads();
-    fwd_pass_fixed<11, MODE>(sm, nullptr, cc, fr.tw, q, q2, fr.q, fr.in.r1, fr.epi);
-    __syncthreads();
-    fwd_pass_fixed<8, MODE>(sm, nullptr, cc, fr.tw, q, q2, fr.q, fr.in.r1, fr.epi);
-    __syncwarp();
-    fwd_pass_fixed<5, MODE>(sm, nullptr, cc, fr.tw, q, q2, fr.q, fr.in.r1, fr.epi);
-    __syncwarp();
-    fwd_pass_fixed<2, MODE, PLAIN>(sm, fr.dst + (size_t)c * (2 * kHalfLoc), cc, fr.tw, q, q2, fr.q, fr.in.r1, fr.epi);
-}
-
-template <int LOGC, bool PLAIN>
-__global__ void __launch_bounds__(256, kNttMinBlocks) ntt_fwd_fixed_kernel(const NttK a)
-{
-    extern __shared__ __align__(16) u64 sm[];
-    FwdRow fr;
-    if (!fwd_row_setup(a, blockIdx.x >> LOGC, fr)) return;
-    unsigned c = 0;
-    if constexpr (LOGC > 0) {
-        c = cg::this_cluster().block_rank();
-        cg::this_cluster().barrier_arrive();
-        const size_t off = (size_t)c * (2 * kHalfLoc);
-        if (fr.epi.aux) fr.epi.aux += off;
-        if (fr.epi.add) fr.epi.add += off;
-        if (fr.epi.mul0) { fr.epi.mul0 += off; fr.epi.mul1 += off; }
-    }
-    switch (fr.mode) {
-    case kF64: fwd_body_fixed<LOGC, kF64, PLAIN>(sm, fr, c); break;
-    case kF64Tight: fwd_body_fixed<LOGC, kF64Tight, PLAIN>(sm, fr, c); break;
-    case kIntLazy: fwd_body_fixed<LOGC, kIntLazy, PLAIN>(sm, fr, c); break;
-    default: fwd_body_fixed<LOGC, kIntStrict, PLAIN>(sm, fr, c); break;
-    }
-}
-
-// three inverse stages starting at distance 2^LOGT
-template <int LOGT, int IM>
-LB_D void inv_pass_fixed(u64 *sm, const u64 *gsrc, const unsigned cc, const ulonglong2 *itw, const u64 q, const u64 q2, const bool reduce)
-{
-    constexpr bool WIDE = LOGT + 3 > 10, OPENING = LOGT == 0;
-    for (int it = 0; it < 4; ++it) {
-        const int g = fixed_group<WIDE>(it);
-        const int lo = g & ((1 << LOGT) - 1), hi = g >> LOGT;
-        const int base = (hi << (LOGT + 3)) + lo;
-        u64 *p = sm + sidx(base);
-        u64 v[8];
-        if constexpr (OPENING) {
-            load_contig<8>(v, gsrc + base);
-            if (is_inv_f64(IM)) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = bits_of(f64_from_u52(v[i]));
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = p[pad_off<LOGT>(i)];
-        }
-        if ((IM == kInvF64 && reduce && !OPENING) || IM == kInvF64Tight) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = bits_of(f64_centre(f64_of(v[i]), f64_of(q), f64_of(q2)));
-        }
-        inv_core<3, false, IM>(v, itw, (cc << (12 - LOGT)) + (hi << 2), q, q2, 0, 0, 0, 0);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) p[pad_off<LOGT>(i)] = v[i];
-    }
-}
-
-template <int LOGC, int IM>
-LB_D void inv_last_fixed(u64 *sm, u64 *dst, const unsigned c, const ulonglong2 *itw, const u64 q, const u64 q2, const u64 cn,
-                         const u64 cns, const u64 cw, const u64 cws, const bool reduce)
-{
-    constexpr int F = LOGC + 1, R0 = 1 << F, COLS = kHalfLoc >> LOGC;
-    const uint32_t sbase = smem_addr(sm);
-    for (int col = threadIdx.x; col < COLS; col += 256) {
-        const int j = c * COLS + col;
-        const int s0 = sidx(j);
-        u64 v[R0];
-        if constexpr (LOGC == 0) {
-            v[0] = sm[s0];
-            v[1] = sm[s0 + kHalfLocPad];
-        } else {
-#pragma unroll
-            for (int r = 0; r < (1 << LOGC); ++r) {
-                const uint32_t ra = map_to_cta(sbase + 8u * s0, r);
-                v[2 * r] = ld_cluster(ra);
-                v[2 * r + 1] = ld_cluster(ra + 8u * kHalfLocPad);
-            }
-        }
-        if ((IM == kInvF64 && reduce) || IM == kInvF64Tight) {
-#pragma unroll
-            for (int k = 0; k < R0; ++k) v[k] = bits_of(f64_centre(f64_of(v[k]), f64_of(q), f64_of(q2)));
-        }
-        inv_core<F, true, IM>(v, itw, 1u << LOGC, q, q2, cn, cns, cw, cws);
-#pragma unroll
-        for (int k = 0; k < R0; ++k) dst[j + k * kHalfLoc] = v[k];
-    }
-}
-
-template <int LOGC, int IM>
-LB_D void inv_body_fixed(u64 *sm, const u64 *src, u64 *dst, const unsigned c, const ulonglong2 *itw, const u64 qi, const u64 cn_i,
-                         const u64 cns_i, const u64 cw_i, const u64 cws_i)
-{
-    const InvConst k = inv_constants(IM, qi, cn_i, cns_i, cw_i, cws_i);
-    const u64 q = k.q, q2 = k.q2;
-    const unsigned cc = (1u << LOGC) + c;
-    F64Run run(qi);
-    const bool r0 = run.before(3), r1 = run.before(3), r2 = run.before(3), r3 = run.before(3), r4 = run.before(LOGC + 1);
-    (void)r0; // the opening pass reads canonical residues
-    inv_pass_fixed<0, IM>(sm, src + (size_t)c * (2 * kHalfLoc), cc, itw, q, q2, false);
-    __syncwarp();
-    inv_pass_fixed<3, IM>(sm, nullptr, cc, itw, q, q2, r1);
-    __syncwarp();
-    inv_pass_fixed<6, IM>(sm, nullptr, cc, itw, q, q2, r2);
-    __syncthreads();
-    inv_pass_fixed<9, IM>(sm, nullptr, cc, itw, q, q2, r3);
-    if constexpr (LOGC > 0) cg::this_cluster().sync(); // every local transform of the cluster is in shared memory
-    else __syncthreads();
-    inv_last_fixed<LOGC, IM>(sm, dst, c, itw, q, q2, k.cn, k.cns, k.cw, k.cws, r4);
-    if constexpr (LOGC > 0) cg::this_cluster().sync(); // shared memory stays alive until every peer has read it
-}
-
-template <int LOGC>
-__global__ void __launch_bounds__(256, kNttMinBlocks) ntt_inv_fixed_kernel(const NttK a)
-{
-    extern __shared__ __align__(16) u64 sm[];
-    const int row = blockIdx.x >> LOGC;
-    const int grp = row / a.per_group, rr = row - grp * a.per_group;
-    if (rr >= a.skip_lo && rr < a.skip_hi) return;
-    const int tbl = rr < a.size_l ? rr + a.tbl_off : a.size_Q + (rr - a.size_l);
-    const ModConst mc = a.mc[tbl];
-    const int logN = a.logN;
-    const ulonglong2 *itw = a.tw + ((size_t)tbl << logN);
-    const int go = grp / a.split, gi = grp - go * a.split;
-    const u64 *src = a.src + (((size_t)go * a.src_outer + (size_t)gi * a.src_group_stride + rr + a.src_row_off) << logN);
-    u64 *dst = a.dst + (((size_t)go * a.dst_outer + (size_t)gi * a.dst_group_stride + rr) << logN);
-    u64 cn = mc.ninv, cns = mc.ninvs, cw = mc.iw1n, cws = mc.iw1ns;
-    if (a.fold) {
-        const u64 *f = a.fold + 4 * rr;
-        cn = f[0]; cns = f[1]; cw = f[2]; cws = f[3];
-    }
-    unsigned c = 0;
-    if constexpr (LOGC > 0) c = cg::this_cluster().block_rank();
-    if (mc.q < kF64PrimeLimit) inv_body_fixed<LOGC, kInvF64>(sm, src, dst, c, itw, mc.q, cn, cns, cw, cws);
-    else if (mc.q < kF64TightPrimeLimit) inv_body_fixed<LOGC, kInvF64Tight>(sm, src, dst, c, itw, mc.q, cn, cns, cw, cws);
-    else inv_body_fixed<LOGC, kInvInt>(sm, src, dst, c, itw, mc.q, cn, cns, cw, cws);
-}
+namespace lb {
 
 // ---- launchers ------------------------------------------------------------------------
 
@@ -1049,23 +696,26 @@ static PassPlan plan_passes(int logn_loc, bool forward)
     return pl;
 }
 
+static bool plain_input(const NttK &k)
+{
+    return k.bconv_n == 0 && k.digit_alpha == 0 && !k.presub && !k.esmall && !k.small && !k.aux && !k.mul2;
+}
+
+static const char *kernel_label(bool forward, const NttK &k)
+{
+    return !forward ? "ntt_inv_kernel" : plain_input(k) ? "ntt_fwd_kernel(plain input)" : "ntt_fwd_kernel(fused input)";
+}
+
+// rings below 4096 points (LOGC == 0) and of 131072 points (LOGC == 4)
 template <int LOGC>
-static int launch(bool forward, bool fixed, const NttK &k, int rows, size_t smem, cudaStream_t stream, double bytes)
+static int launch(bool forward, const NttK &k, int rows, size_t smem, cudaStream_t stream, double bytes)
 {
     auto kern = forward ? ntt_fwd_kernel<LOGC> : ntt_inv_kernel<LOGC>;
-    int which = 0;
-    const bool plain = k.bconv_n == 0 && k.digit_alpha == 0 && !k.presub && !k.esmall && !k.small && !k.aux && !k.mul2;
-    if constexpr (LOGC <= 3) {
-        if (fixed) {
-            kern = !forward ? ntt_inv_fixed_kernel<LOGC> : plain ? ntt_fwd_fixed_kernel<LOGC, true> : ntt_fwd_fixed_kernel<LOGC, false>;
-            which = plain ? 2 : 1;
-        }
-    }
     // function attributes belong to the device the kernel image is loaded on
-    static bool configured[64][2][3] = {};
+    static bool configured[64][2] = {};
     int dev = 0;
     LB_CUDA(cudaGetDevice(&dev));
-    bool &done = configured[dev & 63][forward][which];
+    bool &done = configured[dev & 63][forward];
     if (!done) {
         // largest request any ring degree makes: 8192 points plus one pad word per 16
         LB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024));
@@ -1084,9 +734,56 @@ static int launch(bool forward, bool fixed, const NttK &k, int rows, size_t smem
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    count_launch(!forward ? "ntt_inv_kernel" : plain ? "ntt_fwd_kernel(plain input)" : "ntt_fwd_kernel(fused input)", stream, bytes);
+    count_launch(kernel_label(forward, k), stream, bytes);
     LB_CUDA(cudaLaunchKernelEx(&cfg, kern, k));
     return LB_OK;
+}
+
+// `grid` blocks of `threads`; the kernel may start while its predecessor in the stream drains (see grid_wait)
+static int launch_serial(void (*kern)(const NttK), const NttK &k, long grid, int threads, cudaStream_t stream)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    LB_CUDA(cudaLaunchKernelEx(&cfg, kern, k));
+    return LB_OK;
+}
+
+// Polynomials of one prime that share a block of the row kernels: as many as divide the batch without leaving more than
+// an eighth of the half warps idle.  In mod-up the digits of one ciphertext skip different rows, so there a block takes
+// the same digit of several ciphertexts.
+static void share_rows(NttK &k, int n_groups)
+{
+    k.poly_step = k.digit_alpha > 0 ? k.split : 1;
+    k.n_polys = n_groups / k.poly_step;
+    k.log_polys = 3;
+    while (k.log_polys > 0 && ((k.n_polys + (1 << k.log_polys) - 1) >> k.log_polys << k.log_polys) * 8L > k.n_polys * 9L) --k.log_polys;
+}
+
+template <int A>
+static int launch_twopass(bool forward, NttK &k, int rows, cudaStream_t stream, double bytes)
+{
+    using C = ColShape<A>;
+    share_rows(k, rows / k.per_group);
+    const long col_grid = (long)rows * C::TILES;
+    const long row_grid = (long)((k.n_polys + (1 << k.log_polys) - 1) >> k.log_polys) * k.poly_step * k.per_group << (A - 3 + k.log_polys);
+    const bool plain = plain_input(k);
+    int rc;
+    count_launch(kernel_label(forward, k), stream, bytes);
+    if (forward) {
+        if ((rc = launch_serial(plain ? ntt_fwd_col_kernel<A, true> : ntt_fwd_col_kernel<A, false>, k, col_grid, C::THREADS, stream))) return rc;
+        count_launch(kernel_label(forward, k), stream);
+        return launch_serial(plain ? ntt_fwd_row_kernel<true> : ntt_fwd_row_kernel<false>, k, row_grid, kRowThreads, stream);
+    }
+    if ((rc = launch_serial(ntt_inv_row_kernel, k, row_grid, kRowThreads, stream))) return rc;
+    count_launch(kernel_label(forward, k), stream);
+    return launch_serial(ntt_inv_col_kernel<A>, k, col_grid, C::THREADS, stream);
 }
 
 static int run(Context *ctx, const NttJob &job, bool forward, cudaStream_t stream)
@@ -1130,6 +827,7 @@ static int run(Context *ctx, const NttJob &job, bool forward, cudaStream_t strea
     k.add = job.add;
     k.fold = job.fold;
     k.mul2 = job.mul2;
+    k.mid = job.mid;
     k.presub = job.presub;
     k.esmall = job.esmall;
     k.small = job.small;
@@ -1147,7 +845,6 @@ static int run(Context *ctx, const NttJob &job, bool forward, cudaStream_t strea
     for (int i = 0; i < pl.npass; ++i) k.S[i] = pl.S[i];
     const size_t n_loc = size_t(1) << logn_loc;
     const size_t smem = (n_loc + (n_loc >> 4) + 2) * sizeof(u64);
-    const bool fixed = logn_loc == 13; // rings of 8192 points and more take the fixed-schedule kernels
     // algorithmic bytes of this launch (diagnostics): rows written once; plain rows read once; fused loaders read the
     // group's source rows once per group, plus the rows the epilogue and the prologue fold in
     const double limb = 8.0 * (double)hp.N;
@@ -1165,13 +862,14 @@ static int run(Context *ctx, const NttJob &job, bool forward, cudaStream_t strea
     if (job.presub) bytes += outer * (k.presub_inner < k.split ? k.presub_inner : k.split) * live * limb;
     if (job.esmall) bytes += outer * (double)hp.N;
     if (job.mul2) bytes += out_rows * limb + 2.0 * job.per_group * limb; // a second output row per row, the two fixed rows once
-    switch (logc) {
-    case 0: return launch<0>(forward, fixed, k, rows, smem, stream, bytes);
-    case 1: return launch<1>(forward, fixed, k, rows, smem, stream, bytes);
-    case 2: return launch<2>(forward, fixed, k, rows, smem, stream, bytes);
-    case 3: return launch<3>(forward, fixed, k, rows, smem, stream, bytes);
-    case 4: return launch<4>(forward, fixed, k, rows, smem, stream, bytes);
-    default: set_error("poly_modulus_degree above 65536 is not supported"); return LB_ERR_INVALID_ARG;
+    switch (hp.logN) {
+    case 12: return launch_twopass<4>(forward, k, rows, stream, bytes);
+    case 13: return launch_twopass<5>(forward, k, rows, stream, bytes);
+    case 14: return launch_twopass<6>(forward, k, rows, stream, bytes);
+    case 15: return launch_twopass<7>(forward, k, rows, stream, bytes);
+    case 16: return launch_twopass<8>(forward, k, rows, stream, bytes);
+    case 17: return launch<4>(forward, k, rows, smem, stream, bytes);
+    default: return launch<0>(forward, k, rows, smem, stream, bytes);
     }
 }
 

@@ -1,0 +1,456 @@
+// Two-kernel negacyclic transforms for rings of 4096 to 65536 points (included by ntt.cu).
+//
+// A limb of N = 2^A * 256 coefficients is a matrix of 2^A rows of 256.  The column kernel runs the A stages
+// with spans N/2 .. 256 on tiles of adjacent columns, the row kernel the eight stages with spans 128 .. 1 on single rows;
+// the inverse runs them the other way round.  A thread holds 16 values (8 on the shorter columns) and takes four stages at
+// a time in registers, so a kernel of eight stages exchanges its values once through shared memory:
+//   column kernel  one block barrier; loads and stores are 128-byte segments of a matrix row
+//   row kernel     a row belongs to half a warp, so exchanges need a warp barrier only
+// What bounds them: the integer multiplier / FP64 pipe and the issue slots.  The schedule before this one (one kernel, a
+// cluster of N / 8192 blocks per limb, five radix-8 passes through shared memory) kept issue slots half busy: every
+// pass was a barrier for 256 threads that each walked 32 values, the first one for the whole cluster, and a single
+// limb, a chain of 5 x 4 such steps on N / 8192 SMs, took 20 to 27 us whatever the batch.  Here a limb of 65536 is
+// spread over 4096 threads and a pass over the matrix is a chain of two register steps.  The price is a second trip of the
+// data through L2 / HBM (16 more bytes per coefficient).
+//
+// Code size: the two register groups of a kernel are one loop body, because the bodies of the prime classes (integer and
+// FP64) run side by side on an SM and unrolled in full they missed the instruction cache (2 stalls per issue).  Twiddles are
+// stored in the order the groups read them (twiddle_slot in params.h).
+#pragma once
+#include "ntt_stages.cuh"
+
+namespace lb {
+
+constexpr int kRowLog = 8, kRowThreads = 128, kRowsPerCta = kRowThreads / 16; // half warps per block of the row kernels
+constexpr int kRowPad = 272; // a row in shared memory: one spare word per 16
+
+// shape of the column kernel for 2^A rows: first S1 stages, then S2; 2^S1 values and 2^S2 threads per column
+template <int A>
+struct ColShape {
+    static constexpr int S1 = column_first_stages(A), S2 = A - S1;
+    static constexpr int V = 1 << S1, TPC = 1 << S2;
+    static constexpr int THREADS = A >= 7 ? 256 : 128;
+    static constexpr int COLS = THREADS / TPC; // 128, 32, 16, 32, 16 columns for A = 4 .. 8
+    static constexpr int TILES = 256 / COLS;   // blocks per limb
+    static constexpr int G = 1 << (S1 - S2);   // register groups of the second part per thread (S2 > 0)
+};
+
+// a kernel launched with programmatic stream serialisation may start before its predecessor has finished: nothing
+// is read or written before this
+LB_D void grid_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// the transform's input at column-kernel positions j + (k << LOGST), k < V (see FwdIn)
+template <int V, int LOGST, bool PLAIN>
+LB_D void col_load(u64 (&v)[V], const FwdIn &in, const int j)
+{
+    const u64 q = in.q;
+    if (PLAIN || (in.n == 0 && in.sub == nullptr && in.small == nullptr)) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = in.src[j + (k << LOGST)];
+        return;
+    }
+    if (in.small) {
+        // the small polynomial of an encryption as signed bytes, the same for every prime
+        int ev[V];
+#pragma unroll
+        for (int k = 0; k < V; ++k) ev[k] = in.small[j + (k << LOGST)];
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = ev[k] < 0 ? q - (u64)(-ev[k]) : (u64)ev[k];
+    } else if (in.n == 1 && in.mat == nullptr) {
+        // One source row reduced into this prime (every conversion of a chain with one special prime).  The branches
+        // on the optional parts stay outside the loops so that all loads of a part are in flight together.
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = in.src[j + (k << LOGST)];
+        if (in.es) {
+            int ev[V];
+#pragma unroll
+            for (int k = 0; k < V; ++k) ev[k] = in.es[j + (k << LOGST)];
+#pragma unroll
+            for (int k = 0; k < V; ++k) {
+                const u64 x = add_mod(v[k], ev[k] < 0 ? in.es_p - (u64)(-ev[k]) : (u64)ev[k], in.es_p);
+                v[k] = sub_mod(barrett64(x, q, in.r1), ev[k] < 0 ? q - (u64)(-ev[k]) : (u64)ev[k], q);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < V; ++k) v[k] = barrett64(v[k], q, in.r1);
+        }
+        if (in.sub) {
+#pragma unroll
+            for (int h = 0; h < V; h += 8) {
+                u64 t[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) t[k] = in.sub[j + ((h + k) << LOGST)];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[h + k] = sub_mod(v[h + k], shoup_mul(t[k], in.sub_w, in.sub_ws, q), q);
+            }
+        }
+    } else if (in.mat != nullptr && in.sub == nullptr) {
+        // base conversion of several source rows: four outputs share one walk over the rows, so four loads are in
+        // flight per row instead of one
+#pragma unroll
+        for (int h = 0; h < V; h += 4) {
+            u128d acc[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] = u128d{0, 0};
+            for (int i = 0; i < in.n; ++i) {
+                const u64 m = __ldg(in.mat + i);
+                const u64 *row = in.src + ((size_t)i << in.logN) + j;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mac_wide(acc[k], row[(h + k) << LOGST], m);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[h + k] = barrett128(acc[k], q, in.r0, in.r1);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = load_in(in, j + (k << LOGST));
+    }
+}
+
+template <int A, int M, bool PLAIN>
+LB_D void col_fwd_body(u64 *sm, const FwdRow &fr, u64 *mid, const int tile)
+{
+    using C = ColShape<A>;
+    const int cl = threadIdx.x & (C::COLS - 1), t = threadIdx.x / C::COLS;
+    const int col = tile * C::COLS + cl;
+    const TpPrime p = tp_prime<M>(fr.q);
+    const ulonglong2 *tw = fr.tw;
+    u64 v[C::V];
+    col_load<C::V, kRowLog + C::S2, PLAIN>(v, fr.in, (t << kRowLog) + col);
+#pragma unroll
+    for (int k = 0; k < C::V; ++k) v[k] = tp_load<M>(v[k]);
+    if constexpr (C::S1 == C::S2) {
+        const ulonglong2 *tg = tw + 1;
+#pragma unroll 1
+        for (int half = 0;; ++half) {
+            tp_fwd<C::S1, M>(v, p, [&](const int u, const int b) { return __ldg(tg + (1 << u) - 1 + b); });
+            tp_settle<M>(v, p);
+            if (half) break;
+#pragma unroll
+            for (int k = 0; k < C::V; ++k) sm[((k << C::S2) + t) * C::COLS + cl] = v[k];
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < C::V; ++k) v[k] = sm[((t << C::S2) + k) * C::COLS + cl];
+            tg = tw + (1 << C::S1) + t * ((1 << C::S2) - 1);
+        }
+#pragma unroll
+        for (int k = 0; k < C::V; ++k) mid[(((t << C::S2) + k) << kRowLog) + col] = v[k];
+    } else {
+        tp_fwd<C::S1, M>(v, p, [&](const int u, const int b) { return __ldg(tw + (1 << u) + b); });
+        tp_settle<M>(v, p);
+        if constexpr (C::S2 == 0) {
+#pragma unroll
+            for (int k = 0; k < C::V; ++k) mid[(k << kRowLog) + col] = v[k];
+        } else {
+#pragma unroll
+            for (int k = 0; k < C::V; ++k) sm[((k << C::S2) + t) * C::COLS + cl] = v[k];
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < C::G; ++i) {
+                const int g = t + i * C::TPC;
+                const ulonglong2 *tg = tw + (1 << C::S1) + g * ((1 << C::S2) - 1);
+                u64 w[1 << C::S2];
+#pragma unroll
+                for (int k = 0; k < (1 << C::S2); ++k) w[k] = sm[((g << C::S2) + k) * C::COLS + cl];
+                tp_fwd<C::S2, M>(w, p, [&](const int u, const int b) { return __ldg(tg + (1 << u) - 1 + b); });
+                tp_settle<M>(w, p);
+#pragma unroll
+                for (int k = 0; k < (1 << C::S2); ++k) mid[(((g << C::S2) + k) << kRowLog) + col] = w[k];
+            }
+        }
+    }
+}
+
+template <int A, bool PLAIN>
+__global__ void __launch_bounds__(ColShape<A>::THREADS, ColShape<A>::THREADS == 256 ? 3 : 6) ntt_fwd_col_kernel(const __grid_constant__ NttK a)
+{
+    using C = ColShape<A>;
+    __shared__ __align__(16) u64 sm[C::S2 ? C::V * C::THREADS : 1];
+    grid_wait();
+    const int row = blockIdx.x / C::TILES, tile = blockIdx.x % C::TILES;
+    FwdRow fr;
+    if (!fwd_row_setup(a, row, fr)) return;
+    u64 *mid = a.mid ? a.mid + ((size_t)row << a.logN) : fr.dst;
+    switch (tp_fwd_mode(fr.q)) {
+    case kTpF64: col_fwd_body<A, kTpF64, PLAIN>(sm, fr, mid, tile); break;
+    case kTpF64Tight: col_fwd_body<A, kTpF64Tight, PLAIN>(sm, fr, mid, tile); break;
+    case kTpNear: col_fwd_body<A, kTpNear, PLAIN>(sm, fr, mid, tile); break;
+    case kTpLazy: col_fwd_body<A, kTpLazy, PLAIN>(sm, fr, mid, tile); break;
+    default: col_fwd_body<A, kTpStrict, PLAIN>(sm, fr, mid, tile); break;
+    }
+}
+
+// Which limb row and which matrix row a half warp of a row kernel works on.  The eight half warps of a block take
+// 2^log_polys polynomials of the same prime times 8 / 2^log_polys matrix rows: polynomials that share a matrix row share its
+// 510 twiddles (4 KB of table against 2 KB of data per row), which then come from L1 instead of L2.
+struct RowPlace {
+    int rr, grp, r; // limb within its group (the same for the whole block), group (n_groups or more: nothing to do), matrix row
+};
+LB_D RowPlace row_place(const NttK &a)
+{
+    const int h = threadIdx.x >> 4, log_tiles = a.logN - kRowLog - 3 + a.log_polys;
+    const int tile = blockIdx.x & ((1 << log_tiles) - 1);
+    int rest = blockIdx.x >> log_tiles;
+    RowPlace w;
+    w.rr = rest % a.per_group;
+    rest /= a.per_group;
+    const int sub = rest % a.poly_step;
+    w.grp = (((rest / a.poly_step) << a.log_polys) + (h & ((1 << a.log_polys) - 1))) * a.poly_step + sub;
+    w.r = (tile << (3 - a.log_polys)) + (h >> a.log_polys);
+    return w;
+}
+
+// the 16 x 16 values of a matrix row change hands: thread t has (t, k) and gets (k, t)
+LB_D void row_transpose(u64 (&v)[16], u64 *srow, const int t)
+{
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) srow[t + 17 * k] = v[k];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = srow[17 * t + k];
+}
+
+// a thread's twiddles of a row's first (spans 128 .. 16) and second (spans 8 .. 1) register group, 16 entries apart
+LB_D const ulonglong2 *row_twiddles(const ulonglong2 *tw, const int logN, const int r, const int t, const bool second)
+{
+    return second ? tw + (1 << (logN - 4)) + r * 240 + t : tw + (1 << (logN - kRowLog)) + (r >> 4) * 240 + (r & 15);
+}
+
+template <int M, bool PLAIN>
+LB_D void row_fwd_body(u64 *srow, const NttK &a, const RowPlace &w, const ModConst *mc, const ulonglong2 *tw)
+{
+    const int t = threadIdx.x & 15, logN = a.logN;
+    const u64 q = mc->q;
+    const TpPrime p = tp_prime<M>(q);
+    const long go = w.grp / a.split, gi = w.grp - go * a.split;
+    const size_t base = ((size_t)w.r << kRowLog) + t;
+    u64 *const dst = a.dst + ((size_t)(go * a.dst_outer + gi * a.dst_group_stride + w.rr) << logN) + base;
+    const u64 *const mid = a.mid ? a.mid + ((size_t)((long)w.grp * a.per_group + w.rr) << logN) + base : dst;
+    u64 v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = mid[16 * k];
+    const ulonglong2 *tg = row_twiddles(tw, logN, w.r, t, false);
+#pragma unroll 1
+    for (int half = 0;; ++half) {
+        tp_fwd<4, M>(v, p, [&](const int u, const int b) { return __ldg(tg + 16 * ((1 << u) - 1 + b)); });
+        if (half) break;
+        tp_settle<M>(v, p);
+        row_transpose(v, srow, t);
+        tg = row_twiddles(tw, logN, w.r, t, true);
+    }
+    const u64 r1 = mc->r1;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = tp_canon<M>(v[k], p, r1);
+    row_transpose(v, srow, t); // back to neighbouring threads on neighbouring coefficients
+    if (!PLAIN && a.aux) {
+        const u64 *aux = a.aux + ((size_t)(go * a.aux_outer + gi * a.aux_group_stride + w.rr) << logN) + base;
+        const u64 *add = a.add1 && gi == 1 ? a.add1 + ((size_t)(go * a.add1_outer + w.rr) << logN) + base
+                         : a.add && gi < a.add_inner ? a.add + ((size_t)(go * a.add_outer + gi * a.add_group_stride + w.rr) << logN) + base
+                                                     : nullptr;
+        const u64 scal = a.scal[w.rr], scal_s = a.scal_s[w.rr];
+#pragma unroll
+        for (int h = 0; h < 16; h += 8) {
+            u64 x[8], y[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = aux[16 * (h + k)];
+            if (add) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) y[k] = add[16 * (h + k)];
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[h + k] = shoup_mul(sub_mod(x[k], v[h + k], q), scal, scal_s, q);
+            if (add) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[h + k] = add_mod(v[h + k], y[k], q);
+            }
+        }
+    }
+    if (!PLAIN && a.mul2) {
+        const u64 *mul0 = a.mul2 + ((size_t)w.rr << logN) + base, *mul1 = mul0 + ((size_t)a.per_group << logN);
+        u64 *const dst1 = dst + ((size_t)a.per_group << logN);
+        const u64 m0 = mc->r0;
+#pragma unroll
+        for (int h = 0; h < 16; h += 8) {
+            u64 x[8], y[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                x[k] = mul0[16 * (h + k)];
+                y[k] = mul1[16 * (h + k)];
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                dst1[16 * (h + k)] = mul_mod(v[h + k], y[k], q, m0, r1);
+                v[h + k] = mul_mod(v[h + k], x[k], q, m0, r1);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) dst[16 * k] = v[k];
+}
+
+LB_D int row_table(const NttK &a, const int rr) { return rr < a.size_l ? rr + a.tbl_off : a.size_Q + (rr - a.size_l); }
+
+template <bool PLAIN>
+__global__ void __launch_bounds__(kRowThreads, 6) ntt_fwd_row_kernel(const __grid_constant__ NttK a)
+{
+    __shared__ __align__(16) u64 sm[kRowsPerCta * kRowPad];
+    grid_wait();
+    const RowPlace w = row_place(a);
+    if (w.grp >= a.n_polys * a.poly_step || (w.rr >= a.skip_lo && w.rr < a.skip_hi)) return;
+    if (a.digit_alpha > 0) { // the digit's own limbs stay in NTT form
+        const int s = (w.grp % a.split) * a.digit_alpha;
+        if (w.rr >= s && w.rr < min(s + a.digit_alpha, a.size_l)) return;
+    }
+    const int tbl = row_table(a, w.rr);
+    const ModConst *mc = a.mc + tbl;
+    const ulonglong2 *tw = a.tw + ((size_t)tbl << a.logN);
+    u64 *srow = sm + (threadIdx.x >> 4) * kRowPad;
+    switch (tp_fwd_mode(mc->q)) {
+    case kTpF64: row_fwd_body<kTpF64, PLAIN>(srow, a, w, mc, tw); break;
+    case kTpF64Tight: row_fwd_body<kTpF64Tight, PLAIN>(srow, a, w, mc, tw); break;
+    case kTpNear: row_fwd_body<kTpNear, PLAIN>(srow, a, w, mc, tw); break;
+    case kTpLazy: row_fwd_body<kTpLazy, PLAIN>(srow, a, w, mc, tw); break;
+    default: row_fwd_body<kTpStrict, PLAIN>(srow, a, w, mc, tw); break;
+    }
+}
+
+// ---- inverse ---------------------------------------------------------------------------
+
+// Where an inverse transform's row comes from and goes to
+struct InvRow {
+    const u64 *src;
+    u64 *dst;
+    const ulonglong2 *itw;
+    u64 q, cn, cns, cw, cws;
+};
+
+LB_D bool inv_row_setup(const NttK &a, const int row, InvRow &r)
+{
+    const int grp = row / a.per_group, rr = row - grp * a.per_group;
+    if (rr >= a.skip_lo && rr < a.skip_hi) return false;
+    const int tbl = rr < a.size_l ? rr + a.tbl_off : a.size_Q + (rr - a.size_l);
+    const ModConst mc = a.mc[tbl];
+    const int go = grp / a.split, gi = grp - go * a.split;
+    r.q = mc.q;
+    r.itw = a.tw + ((size_t)tbl << a.logN);
+    r.src = a.src + (((size_t)go * a.src_outer + (size_t)gi * a.src_group_stride + rr + a.src_row_off) << a.logN);
+    r.dst = a.dst + (((size_t)go * a.dst_outer + (size_t)gi * a.dst_group_stride + rr) << a.logN);
+    r.cn = mc.ninv; r.cns = mc.ninvs; r.cw = mc.iw1n; r.cws = mc.iw1ns;
+    if (a.fold) {
+        const u64 *f = a.fold + 4 * rr;
+        r.cn = f[0]; r.cns = f[1]; r.cw = f[2]; r.cws = f[3];
+    }
+    return true;
+}
+
+template <int M>
+LB_D void row_inv_body(u64 *srow, const NttK &a, const RowPlace &w, const u64 q, const ulonglong2 *tw)
+{
+    const int t = threadIdx.x & 15, logN = a.logN;
+    const TpPrime p = tp_prime<M>(q);
+    const long go = w.grp / a.split, gi = w.grp - go * a.split;
+    const size_t base = ((size_t)w.r << kRowLog) + t;
+    const u64 *const src = a.src + ((size_t)(go * a.src_outer + gi * a.src_group_stride + w.rr + a.src_row_off) << logN) + base;
+    u64 *const dst = a.dst + ((size_t)(go * a.dst_outer + gi * a.dst_group_stride + w.rr) << logN) + base;
+    const TpClose none = {0, 0, 0, 0};
+    u64 v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = src[16 * k];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = tp_load<M>(v[k]);
+#pragma unroll 1
+    for (int half = 1; half >= 0; --half) {
+        row_transpose(v, srow, t);
+        const ulonglong2 *tg = row_twiddles(tw, logN, w.r, t, half);
+        tp_inv<4, M, false>(v, p, [&](const int u, const int b) { return __ldg(tg + 16 * ((1 << (3 - u)) - 1 + b)); }, none);
+        tp_settle<M>(v, p);
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) dst[16 * k] = v[k];
+}
+
+__global__ void __launch_bounds__(kRowThreads, 6) ntt_inv_row_kernel(const __grid_constant__ NttK a)
+{
+    __shared__ __align__(16) u64 sm[kRowsPerCta * kRowPad];
+    grid_wait();
+    const RowPlace w = row_place(a);
+    if (w.grp >= a.n_polys * a.poly_step || (w.rr >= a.skip_lo && w.rr < a.skip_hi)) return;
+    const int tbl = row_table(a, w.rr);
+    const u64 q = a.mc[tbl].q;
+    const ulonglong2 *tw = a.tw + ((size_t)tbl << a.logN);
+    u64 *srow = sm + (threadIdx.x >> 4) * kRowPad;
+    switch (tp_inv_mode(q)) {
+    case kTpF64: row_inv_body<kTpF64>(srow, a, w, q, tw); break;
+    case kTpF64Tight: row_inv_body<kTpF64Tight>(srow, a, w, q, tw); break;
+    case kTpNear: row_inv_body<kTpNear>(srow, a, w, q, tw); break;
+    default: row_inv_body<kTpStrict>(srow, a, w, q, tw); break;
+    }
+}
+
+template <int A, int M>
+LB_D void col_inv_body(u64 *sm, const InvRow &ir, const int tile)
+{
+    using C = ColShape<A>;
+    const int cl = threadIdx.x & (C::COLS - 1), t = threadIdx.x / C::COLS;
+    const int col = tile * C::COLS + cl;
+    const TpPrime p = tp_prime<M>(ir.q);
+    const TpClose close = tp_close<M>(ir.q, ir.cn, ir.cns, ir.cw, ir.cws);
+    const ulonglong2 *tw = ir.itw;
+    u64 *dst = ir.dst;
+    u64 v[C::V];
+    if constexpr (C::S2 == 0) {
+#pragma unroll
+        for (int k = 0; k < C::V; ++k) v[k] = dst[(k << kRowLog) + col];
+        if (M == kTpF64) { // small primes are brought back once per transform
+#pragma unroll
+            for (int k = 0; k < C::V; ++k) v[k] = tp_centre<M>(v[k], p);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < C::G; ++i) {
+            const int g = t + i * C::TPC;
+            const ulonglong2 *tg = tw + (1 << C::S1) + g * ((1 << C::S2) - 1);
+            u64 w[1 << C::S2];
+#pragma unroll
+            for (int k = 0; k < (1 << C::S2); ++k) w[k] = dst[(((g << C::S2) + k) << kRowLog) + col];
+            if (M == kTpF64) {
+#pragma unroll
+                for (int k = 0; k < (1 << C::S2); ++k) w[k] = tp_centre<M>(w[k], p);
+            }
+            tp_inv<C::S2, M, false>(w, p, [&](const int u, const int b) { return __ldg(tg + (1 << (C::S2 - 1 - u)) - 1 + b); }, close);
+            tp_settle<M>(w, p);
+#pragma unroll
+            for (int k = 0; k < (1 << C::S2); ++k) sm[((g << C::S2) + k) * C::COLS + cl] = w[k];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < C::V; ++k) v[k] = sm[((k << C::S2) + t) * C::COLS + cl];
+    }
+    tp_inv<C::S1, M, true>(v, p, [&](const int u, const int b) { return __ldg(tw + (1 << (C::S1 - 1 - u)) + b); }, close);
+#pragma unroll
+    for (int k = 0; k < C::V; ++k) dst[((((k << C::S2) + t)) << kRowLog) + col] = v[k];
+}
+
+template <int A>
+__global__ void __launch_bounds__(ColShape<A>::THREADS, ColShape<A>::THREADS == 256 ? 3 : 6) ntt_inv_col_kernel(const __grid_constant__ NttK a)
+{
+    using C = ColShape<A>;
+    __shared__ __align__(16) u64 sm[C::S2 ? C::V * C::THREADS : 1];
+    grid_wait();
+    const int row = blockIdx.x / C::TILES, tile = blockIdx.x % C::TILES;
+    InvRow ir;
+    if (!inv_row_setup(a, row, ir)) return;
+    switch (tp_inv_mode(ir.q)) {
+    case kTpF64: col_inv_body<A, kTpF64>(sm, ir, tile); break;
+    case kTpF64Tight: col_inv_body<A, kTpF64Tight>(sm, ir, tile); break;
+    case kTpNear: col_inv_body<A, kTpNear>(sm, ir, tile); break;
+    default: col_inv_body<A, kTpStrict>(sm, ir, tile); break;
+    }
+}
+
+} // namespace lb

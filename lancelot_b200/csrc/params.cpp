@@ -156,10 +156,11 @@ bool HostParams::init(int logN_, const std::vector<u64> &moduli, int size_P_, co
         for (u64 i = 0; i < N; ++i) {
             const uint32_t r = bit_reverse((uint32_t)i, logN);
             if (r == 1) ipw_at_1 = ipw;
-            t[2 * r] = h_twiddle_value(pw, p);
-            t[2 * r + 1] = h_twiddle_quot(pw, p);
-            it[2 * r] = h_twiddle_value(ipw, p);
-            it[2 * r + 1] = h_twiddle_quot(ipw, p);
+            const u64 s = twiddle_slot(r, logN);
+            t[2 * s] = h_twiddle_value(pw, p);
+            t[2 * s + 1] = h_twiddle_quot(pw, p);
+            it[2 * s] = h_twiddle_value(ipw, p);
+            it[2 * s + 1] = h_twiddle_quot(ipw, p);
             pw = h_mulmod(pw, psi[m], p);
             ipw = h_mulmod(ipw, ipsi, p);
         }

@@ -29,6 +29,26 @@ uint32_t galois_elt_from_step(int step, u64 N);
 // (cahel-main/include/util/hestdparms.h), 0 when N is outside the table.
 int max_bit_count_tc128(u64 N);
 
+// Where entry i = m + k of a twiddle table is stored.  The transforms of 4096 to 65536 points (ntt_twopass.cuh) run four
+// register groups of stages: S1 and S2 stages on columns, four and four on rows.  The entries a thread needs for one
+// group are numbered s = 2^u - 1 + b (block b at stage u of the group) and stored next to each other (column groups) or 16
+// apart, with the threads of a row (last group) or 16 neighbouring rows (third group) side by side.  Every other ring keeps
+// entry i at index i.
+constexpr int column_first_stages(int A) { return A >= 7 || A == 4 ? 4 : 3; } // S1 of A column stages
+inline u64 twiddle_slot(u64 i, int logN)
+{
+    if (logN < 12 || logN > 16) return i;
+    const int A = logN - 8, S1 = column_first_stages(A), S2 = A - S1;
+    const u64 one = 1;
+    if (i < one << S1) return i;
+    const int first = i < one << A ? S1 : i < one << (A + 4) ? A : A + 4; // the group's first stage
+    int u = 0;
+    while (i >= one << (first + u + 1)) ++u;
+    const u64 k = i - (one << (first + u)), s = (one << u) - 1 + (k & ((one << u) - 1)), g = k >> u;
+    if (first == S1 && S2 > 0) return (one << S1) + g * ((one << S2) - 1) + s;
+    return (one << first) + (g >> 4) * 240 + s * 16 + (g & 15);
+}
+
 // Constants of one data level (size_l data limbs in use).
 struct LevelConst {
     int size_l = 0, beta = 0;
@@ -50,7 +70,7 @@ struct HostParams {
     int size_QP = 0, size_Q = 0, size_P = 0;
     std::vector<u64> q, psi;
     std::vector<ModConst> mc;             // [size_QP]
-    std::vector<u64> tw, itw;             // [size_QP][N][2]  (value, Shoup quotient or, below 2^50, the double value / q), index m + k
+    std::vector<u64> tw, itw;             // [size_QP][N][2]  (value, Shoup quotient; below 2^50 both as doubles), entry m + k at twiddle_slot(m + k)
     std::vector<uint32_t> galois_elts;    // as given by the caller
     std::vector<uint32_t> perm;           // [n_elts][N]
     std::vector<LevelConst> level;        // index = size_l (1..size_Q); [0] unused
