@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(256) compose_kernel(cplx *__restrict__ out, co
             const ModConst m = mc[r];
             const u64 t = coef[((size_t)r << logN) + ((size_t)id << ratio_log)];
             u64 acc = 0;
-            for (int s = 0; s < r; ++s) acc = add_mod(acc, mul_mod(barrett64(v[s], m.q, m.r1), cc.radix_mod[r][s], m.q, m.r0, m.r1), m.q);
+            for (int s = 0; s < r; ++s) acc = add_mod(acc, mul_mod(barrett64(v[s], m.q, m.r1), cc.radix_mod[r][s], m), m.q);
             v[r] = shoup_mul(sub_mod(t, acc, m.q), cc.ginv[r], cc.ginv_s[r], m.q);
         }
         u64 x[kMaxComposeLimbs + 1];

@@ -127,32 +127,24 @@ struct IpArgs {
 // (15 steps x 2 digits of key per ciphertext: 17 GB of L2 reads per launch at 190 ciphertexts).
 template <bool GATHER>
 constexpr int ip_cts() { return GATHER ? 4 : 2; }
-template <bool GATHER>
-__global__ void __launch_bounds__(kKsThreads) inner_product_kernel(const u64 *__restrict__ digits, const u64 *__restrict__ own,
-                                                                   const long own_stride, u64 *__restrict__ cx,
-                                                                   const ModConst *__restrict__ mc, const IpArgs args, const int logN,
-                                                                   const int L, const int LP, const int size_Q, const int size_QP,
-                                                                   const int alpha, const int beta, const int batch)
+template <bool GATHER, uint32_t KIND>
+LB_D void inner_product_body(const u64 *__restrict__ digits, const u64 *__restrict__ own, const long own_stride, u64 *__restrict__ cx,
+                             const ModConst &m, const IpArgs &args, const int logN, const int L, const int LP, const int tbl,
+                             const int size_QP, const int alpha, const int beta, const int batch)
 {
     constexpr int V = GATHER ? 1 : 2, B = ip_cts<GATHER>();
     const long per_ct = (long)LP << logN;
     const int r = blockIdx.y;
-    const int tbl = r < L ? r : size_Q + (r - L);
-    const ModConst m = mc[tbl];
     const int own_digit = r < L ? r / alpha : -1;
     const long n = 1L << logN;
     for (long b0 = (long)blockIdx.z * B; b0 < batch; b0 += (long)gridDim.z * B) {
         const int nb = (int)min((long)B, batch - b0);
         for (long k = ((long)blockIdx.x * blockDim.x + threadIdx.x) * V; k < n; k += (long)gridDim.x * blockDim.x * V) {
             u128d a0[B][V], a1[B][V];
-            u64 r0[B][V], r1[B][V];
 #pragma unroll
             for (int c = 0; c < B; ++c) {
 #pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    a0[c][v] = a1[c][v] = u128d{0, 0};
-                    r0[c][v] = r1[c][v] = 0;
-                }
+                for (int v = 0; v < V; ++v) a0[c][v] = a1[c][v] = u128d{0, 0};
             }
             // one term = one digit of one step; the operands of term t + 1 are requested before term t is multiplied,
             // so the loads of a term have the whole multiply-accumulate of its predecessor to arrive in
@@ -211,9 +203,8 @@ __global__ void __launch_bounds__(kKsThreads) inner_product_kernel(const u64 *__
                     for (int c = 0; c < B; ++c) {
 #pragma unroll
                         for (int v = 0; v < V; ++v) {
-                            r0[c][v] = add_mod(r0[c][v], barrett128(a0[c][v], m.q, m.r0, m.r1), m.q);
-                            r1[c][v] = add_mod(r1[c][v], barrett128(a1[c][v], m.q, m.r0, m.r1), m.q);
-                            a0[c][v] = a1[c][v] = u128d{0, 0};
+                            a0[c][v] = u128d{reduce_wide<KIND>(a0[c][v], m), 0};
+                            a1[c][v] = u128d{reduce_wide<KIND>(a1[c][v], m), 0};
                         }
                     }
                     pending = 0;
@@ -223,23 +214,38 @@ __global__ void __launch_bounds__(kKsThreads) inner_product_kernel(const u64 *__
 #pragma unroll
             for (int c = 0; c < B; ++c) {
                 if (c < nb) {
+                    u64 r0[V], r1[V];
                     u64 *o0 = cx + 2 * (b0 + c) * per_ct + ((long)r << logN) + k, *o1 = o0 + per_ct;
 #pragma unroll
                     for (int v = 0; v < V; ++v) {
-                        r0[c][v] = add_mod(r0[c][v], barrett128(a0[c][v], m.q, m.r0, m.r1), m.q);
-                        r1[c][v] = add_mod(r1[c][v], barrett128(a1[c][v], m.q, m.r0, m.r1), m.q);
+                        r0[v] = reduce_wide<KIND>(a0[c][v], m);
+                        r1[v] = reduce_wide<KIND>(a1[c][v], m);
                     }
                     if (GATHER) {
-                        o0[0] = r0[c][0];
-                        o1[0] = r1[c][0];
+                        o0[0] = r0[0];
+                        o1[0] = r1[0];
                     } else {
-                        *reinterpret_cast<ulonglong2 *>(o0) = make_ulonglong2(r0[c][0], r0[c][V - 1]);
-                        *reinterpret_cast<ulonglong2 *>(o1) = make_ulonglong2(r1[c][0], r1[c][V - 1]);
+                        *reinterpret_cast<ulonglong2 *>(o0) = make_ulonglong2(r0[0], r0[V - 1]);
+                        *reinterpret_cast<ulonglong2 *>(o1) = make_ulonglong2(r1[0], r1[V - 1]);
                     }
                 }
             }
         }
     }
+}
+
+template <bool GATHER>
+__global__ void __launch_bounds__(kKsThreads) inner_product_kernel(const u64 *__restrict__ digits, const u64 *__restrict__ own,
+                                                                   const long own_stride, u64 *__restrict__ cx,
+                                                                   const ModConst *__restrict__ mc, const __grid_constant__ IpArgs args,
+                                                                   const int logN, const int L, const int LP, const int size_Q,
+                                                                   const int size_QP, const int alpha, const int beta, const int batch)
+{
+    const int r = blockIdx.y, tbl = r < L ? r : size_Q + (r - L);
+    const ModConst m = mc[tbl];
+    with_wide_kind(m.kind, [&](auto kind) {
+        inner_product_body<GATHER, decltype(kind)::value>(digits, own, own_stride, cx, m, args, logN, L, LP, tbl, size_QP, alpha, beta, batch);
+    });
 }
 
 static int inner_product_steps(Context *ctx, int L, int batch, const u64 *digits, const u64 *own, long own_stride, const IpArgs &args,

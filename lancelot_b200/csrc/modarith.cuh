@@ -6,6 +6,7 @@
 // (cahel-main/src/ntt/fntt_2d.cu:860-866, cahel-main/include/uintmodmath.cuh:112-259).
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 namespace lb {
 
@@ -90,6 +91,33 @@ inline u64 h_fp_quot(u64 w, u64 q)
 // (primes below 2^50 run their butterflies on the FP64 pipe: the power as a double, and its quotient by q)
 inline u64 h_twiddle_value(u64 w, u64 q) { return q < kF64TightPrimeLimit ? h_bits_of(h_centred(w, q)) : w; }
 inline u64 h_twiddle_quot(u64 w, u64 q) { return q < kF64TightPrimeLimit ? h_fp_quot(w, q) : h_shoup(w, q); }
+
+// Per-modulus constants as laid out in device memory (one entry per prime of QP).
+struct alignas(16) ModConst {
+    u64 q;
+    u64 r0, r1;      // floor(2^128 / q), low and high word
+    u64 ninv, ninvs; // N^-1 mod q and its Shoup quotient
+    u64 iw1n, iw1ns; // psi^-bitrev(1) * N^-1 (last inverse stage fused with the scaling)
+    uint32_t kind;   // how 128-bit sums are reduced, one of the three below
+    uint32_t near_d; // kWideNear: 2^60 - q
+    double qd, qi;   // kWideF64: q, 1 / q, 2^32 / q, the residue of 2^64 nearest zero and its quotient by q
+    double qi32, c64, c64q;
+    u64 pad;
+};
+// near 2^60: integer primes with 2^60 - q < 2^28 (what CoeffModulus hands out for 60 bits)
+constexpr u64 kNearTop = u64(1) << 60, kNearSpan = u64(1) << 28;
+enum : uint32_t { kWideBarrett = 0, kWideNear = 1, kWideF64 = 2 };
+inline void h_wide_constants(ModConst &c)
+{
+    c.kind = c.q < kF64TightPrimeLimit && (c.q >> 34) ? kWideF64 : c.q < kNearTop && kNearTop - c.q < kNearSpan ? kWideNear : kWideBarrett;
+    c.near_d = c.kind == kWideNear ? (uint32_t)(kNearTop - c.q) : 0;
+    c.qd = (double)c.q;
+    c.qi = 1.0 / c.qd;
+    c.qi32 = 4294967296.0 * c.qi;
+    c.c64 = h_centred((u64)(((u128)1 << 64) % c.q), c.q);
+    c.c64q = c.c64 / c.qd;
+    c.pad = 0;
+}
 
 #if defined(__CUDACC__)
 // ---- device arithmetic ----------------------------------------------------------------
@@ -235,16 +263,92 @@ LB_D u64 barrett128(u128d z, u64 q, u64 r0, u64 r1)
     return csub(r, q);
 }
 
-LB_D u64 mul_mod(u64 a, u64 b, u64 q, u64 r0, u64 r1) { return barrett128(mul_wide(a, b), q, r0, r1); }
-#endif
+// ---- reductions of products and sums of products ---------------------------------------------------
+// Two classes of primes have cheaper reductions than the two-word Barrett quotient (18 products of 32 x 32 bits):
+//   near 2^60   2^64 = 16 d and 2^60 = d modulo q with d = 2^60 - q < 2^28, so the high half folds onto the low one with
+//               four products;
+//   FP64        2^34 <= q < 2^50: the high half times 2^64 mod q and the quotient of the low half are formed on the
+//               FP64 pipe, which these kernels leave idle otherwise.
+// The reductions, not the products they belong to, were what bounded the element-wise kernels and the inner product.
 
-// Per-modulus constants as laid out in device memory (one entry per prime of QP).
-struct ModConst {
-    u64 q;
-    u64 r0, r1;      // floor(2^128 / q), low and high word
-    u64 ninv, ninvs; // N^-1 mod q and its Shoup quotient
-    u64 iw1n, iw1ns; // psi^-bitrev(1) * N^-1 (last inverse stage fused with the scaling)
-    u64 pad;
-};
+// any 64-bit word -> congruent word below 2^60 + 15 (2^60 - q)
+LB_D u64 near_reduce(const u64 v, const uint32_t d)
+{
+    return (v & (kNearTop - 1)) + (u64)(uint32_t)(v >> 60) * d;
+}
+// any 128-bit word -> congruent word below 2^60 + 15 (2^60 - q).  The first fold leaves 96 bits: (2^64 - 1) 16 d + 2^64 < 2^96;
+// the second 64 and a carry, whose 16 d fit because the wrapped sum is below 2^64 - 16 d.
+LB_D u64 near_fold(const u128d z, const uint32_t d)
+{
+    const uint32_t d16 = d << 4;
+    const u64 p0 = (u64)(uint32_t)z.hi * d16, p1 = (u64)(uint32_t)(z.hi >> 32) * d16;
+    const u128 t = (u128)z.lo + p0 + ((u128)p1 << 32);
+    const u64 lo = (u64)t, p2 = (u64)(uint32_t)(t >> 64) * d16;
+    u64 r = lo + p2;
+    r += r < lo ? d16 : 0u;
+    return near_reduce(r, d);
+}
+
+// x mod q for any 64-bit x as an integer of magnitude at most q / 2 + 2^32, for 2^34 <= q < 2^50.  The quotient, below 2^30, is
+// taken from the upper half of x and read out of the mantissa of 1.5 * 2^52 + quotient.
+LB_D u64 f64_fold64(const u64 x, const ModConst &m)
+{
+    const double xh = __dadd_rn(__hiloint2double(0x43300000, (int)(x >> 32)), -4503599627370496.0);
+    const uint32_t Q = (uint32_t)__double2loint(__fma_rn(xh, m.qi32, 6755399441055744.0));
+    return x - (u64)Q * m.q;
+}
+// a signed integer of magnitude below 2^51 (two's complement) as a double
+LB_D double f64_from_s52(const u64 x) { return __dadd_rn(f64_of(x + 0x4338000000000000ull), -6755399441055744.0); }
+// (hi:lo) mod q as an integer-valued double of magnitude at most 1.3 q, for 2^34 <= q < 2^50 and hi < 2^52:
+// |hi c64 / q| <= 2^51 is the range of the quotient in f64_mulmod
+LB_D double f64_fold(const u128d z, const ModConst &m)
+{
+    const double h = f64_mulmod(f64_from_u52(z.hi), m.c64, m.c64q, m.qd);
+    return __dadd_rn(__dadd_rn(h, f64_of(f64_fold64(z.lo, m) + 0x4338000000000000ull)), -6755399441055744.0);
+}
+
+// (hi:lo) mod q, canonical.  kWideF64 takes hi < 2^52: sums of 2^15 products of residues, or of 64 products of a residue
+// with a 60-bit word.
+template <uint32_t KIND>
+LB_D u64 reduce_wide(const u128d z, const ModConst &m)
+{
+    if (KIND == kWideNear) return csub(near_fold(z, m.near_d), m.q);
+    if (KIND == kWideF64) return f64_canon(f64_fold(z, m), m.qd, m.qi);
+    return barrett128(z, m.q, m.r0, m.r1);
+}
+LB_D u64 reduce_wide(const u128d z, const ModConst &m)
+{
+    if (m.kind == kWideNear) return reduce_wide<kWideNear>(z, m);
+    if (m.kind == kWideF64) return reduce_wide<kWideF64>(z, m);
+    return reduce_wide<kWideBarrett>(z, m);
+}
+
+// canonical product of residues.  FP64: |a b / q| < 2^50, so the quotient is off by at most 0.5 + 2^-2 as in f64_mulmod
+// although its factor b / q is rounded twice.
+template <uint32_t KIND>
+LB_D u64 mul_mod(const u64 a, const u64 b, const ModConst &m)
+{
+    if (KIND == kWideF64) {
+        const double w = f64_from_u52(b);
+        return f64_canon(f64_mulmod(f64_from_u52(a), w, __dmul_rn(w, m.qi), m.qd), m.qd, m.qi);
+    }
+    return reduce_wide<KIND>(mul_wide(a, b), m);
+}
+LB_D u64 mul_mod(const u64 a, const u64 b, const ModConst &m)
+{
+    if (m.kind == kWideNear) return mul_mod<kWideNear>(a, b, m);
+    if (m.kind == kWideF64) return mul_mod<kWideF64>(a, b, m);
+    return mul_mod<kWideBarrett>(a, b, m);
+}
+
+// calls body with the prime's class as a compile-time constant
+template <class F>
+LB_D void with_wide_kind(const uint32_t kind, const F &body)
+{
+    if (kind == kWideNear) body(std::integral_constant<uint32_t, kWideNear>());
+    else if (kind == kWideF64) body(std::integral_constant<uint32_t, kWideF64>());
+    else body(std::integral_constant<uint32_t, kWideBarrett>());
+}
+#endif
 
 } // namespace lb

@@ -283,11 +283,11 @@ LB_D void fwd_pass(u64 *sm, const bool from_global, u64 *gdst, const FwdIn &in, 
                 u64 t[R], w[R];
                 load_contig<R>(t, epi.mul1 + base);
 #pragma unroll
-                for (int i = 0; i < R; ++i) w[i] = mul_mod(v[i], t[i], qi, epi.r0, epi.r1);
+                for (int i = 0; i < R; ++i) w[i] = barrett128(mul_wide(v[i], t[i]), qi, epi.r0, epi.r1);
                 store_contig<R>(w, gdst + epi.dst1_off + base);
                 load_contig<R>(t, epi.mul0 + base);
 #pragma unroll
-                for (int i = 0; i < R; ++i) v[i] = mul_mod(v[i], t[i], qi, epi.r0, epi.r1);
+                for (int i = 0; i < R; ++i) v[i] = barrett128(mul_wide(v[i], t[i]), qi, epi.r0, epi.r1);
             }
             store_contig<R>(v, gdst + base);
         } else {

@@ -20,7 +20,6 @@ namespace lb {
 enum { kTpStrict = 0, kTpLazy = 1, kTpNear = 2, kTpF64Tight = 3, kTpF64 = 4 };
 LB_D constexpr bool tp_f64(const int m) { return m == kTpF64 || m == kTpF64Tight; }
 
-constexpr u64 kNearTop = u64(1) << 60, kNearSpan = u64(1) << 28;
 // primes below 2^42 need no reduction inside a kernel of an inverse transform (sums of at most nine stages)
 constexpr u64 kF64InvPrimeLimit = u64(1) << 42;
 
@@ -55,12 +54,6 @@ LB_D TpPrime tp_prime(const u64 q)
     }
     p.d = (uint32_t)(kNearTop - q);
     return p;
-}
-
-// any 64-bit word -> congruent word below 2^60 + 15 (2^60 - q)
-LB_D u64 near_reduce(const u64 v, const uint32_t d)
-{
-    return (v & (kNearTop - 1)) + (u64)(uint32_t)(v >> 60) * d;
 }
 
 template <int M>

@@ -284,8 +284,8 @@ LB_D void row_fwd_body(u64 *srow, const NttK &a, const RowPlace &w, const ModCon
             }
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                dst1[16 * (h + k)] = mul_mod(v[h + k], y[k], q, m0, r1);
-                v[h + k] = mul_mod(v[h + k], x[k], q, m0, r1);
+                dst1[16 * (h + k)] = barrett128(mul_wide(v[h + k], y[k]), q, m0, r1);
+                v[h + k] = barrett128(mul_wide(v[h + k], x[k]), q, m0, r1);
             }
         }
     }

@@ -173,7 +173,7 @@ bool HostParams::init(int logN_, const std::vector<u64> &moduli, int size_P_, co
         c.ninvs = h_shoup(c.ninv, p);
         c.iw1n = h_mulmod(ipw_at_1, c.ninv, p);
         c.iw1ns = h_shoup(c.iw1n, p);
-        c.pad = 0;
+        h_wide_constants(c);
     }
 
     galois_elts = elts;

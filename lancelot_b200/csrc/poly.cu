@@ -38,12 +38,12 @@ __global__ void __launch_bounds__(kPolyThreads) binary_kernel(const ulonglong2 *
             r.x = sub_mod(x.x, y.x, m.q);
             r.y = sub_mod(x.y, y.y, m.q);
         } else if (OP == OP_MUL) {
-            r.x = mul_mod(x.x, y.x, m.q, m.r0, m.r1);
-            r.y = mul_mod(x.y, y.y, m.q, m.r0, m.r1);
+            r.x = reduce_wide(mul_wide(x.x, y.x), m);
+            r.y = reduce_wide(mul_wide(x.y, y.y), m);
         } else if (OP == OP_REDUCE) {
             // any 64-bit word, e.g. a plain sum of residues, back to its canonical residue
-            r.x = barrett128(u128d{x.x, 0}, m.q, m.r0, m.r1);
-            r.y = barrett128(u128d{x.y, 0}, m.q, m.r0, m.r1);
+            r.x = reduce_wide(u128d{x.x, 0}, m);
+            r.y = reduce_wide(u128d{x.y, 0}, m);
         } else {
             r.x = x.x ? m.q - x.x : 0;
             r.y = x.y ? m.q - x.y : 0;
@@ -75,11 +75,12 @@ int poly_binary(Context *ctx, int op, int size_l, long rows, const u64 *a, const
 
 // ---- tensor product ---------------------------------------------------------------------
 
+template <uint32_t KIND>
 LB_D u64 tensor_mid(u64 a0, u64 b1, u64 a1, u64 b0, const ModConst &m)
 {
     u128d acc = mul_wide(a0, b1);
     mac_wide(acc, a1, b0);
-    return barrett128(acc, m.q, m.r0, m.r1);
+    return reduce_wide<KIND>(acc, m);
 }
 
 __global__ void __launch_bounds__(kPolyThreads) tensor_kernel(const ulonglong2 *__restrict__ a, const ulonglong2 *__restrict__ b,
@@ -94,12 +95,15 @@ __global__ void __launch_bounds__(kPolyThreads) tensor_kernel(const ulonglong2 *
         const ulonglong2 a0 = a[ct * 2 * per_ct + e], a1 = a[ct * 2 * per_ct + per_ct + e];
         const ulonglong2 b0 = b[ct * 2 * per_ct + e], b1 = b[ct * 2 * per_ct + per_ct + e];
         ulonglong2 d0, d1, d2;
-        d0.x = mul_mod(a0.x, b0.x, m.q, m.r0, m.r1);
-        d0.y = mul_mod(a0.y, b0.y, m.q, m.r0, m.r1);
-        d1.x = tensor_mid(a0.x, b1.x, a1.x, b0.x, m);
-        d1.y = tensor_mid(a0.y, b1.y, a1.y, b0.y, m);
-        d2.x = mul_mod(a1.x, b1.x, m.q, m.r0, m.r1);
-        d2.y = mul_mod(a1.y, b1.y, m.q, m.r0, m.r1);
+        with_wide_kind(m.kind, [&](auto kind) {
+            constexpr uint32_t K = decltype(kind)::value;
+            d0.x = reduce_wide<K>(mul_wide(a0.x, b0.x), m);
+            d0.y = reduce_wide<K>(mul_wide(a0.y, b0.y), m);
+            d1.x = tensor_mid<K>(a0.x, b1.x, a1.x, b0.x, m);
+            d1.y = tensor_mid<K>(a0.y, b1.y, a1.y, b0.y, m);
+            d2.x = reduce_wide<K>(mul_wide(a1.x, b1.x), m);
+            d2.y = reduce_wide<K>(mul_wide(a1.y, b1.y), m);
+        });
         out[ct * 3 * per_ct + e] = d0;
         out[ct * 3 * per_ct + per_ct + e] = d1;
         out[ct * 3 * per_ct + 2 * per_ct + e] = d2;
@@ -254,12 +258,15 @@ __global__ void __launch_bounds__(kKrumThreads) krum_accumulate_kernel(const ulo
                 mac_wide(s2x, x1, x1);
                 mac_wide(s2y, y1, y1);
             }
-            r0x = add_mod(r0x, barrett128(s0x, m.q, m.r0, m.r1), m.q);
-            r0y = add_mod(r0y, barrett128(s0y, m.q, m.r0, m.r1), m.q);
-            r1x = add_mod(r1x, barrett128(s1x, m.q, m.r0, m.r1), m.q);
-            r1y = add_mod(r1y, barrett128(s1y, m.q, m.r0, m.r1), m.q);
-            r2x = add_mod(r2x, barrett128(s2x, m.q, m.r0, m.r1), m.q);
-            r2y = add_mod(r2y, barrett128(s2y, m.q, m.r0, m.r1), m.q);
+            with_wide_kind(m.kind, [&](auto kind) {
+                constexpr uint32_t K = decltype(kind)::value;
+                r0x = add_mod(r0x, reduce_wide<K>(s0x, m), m.q);
+                r0y = add_mod(r0y, reduce_wide<K>(s0y, m), m.q);
+                r1x = add_mod(r1x, reduce_wide<K>(s1x, m), m.q);
+                r1y = add_mod(r1y, reduce_wide<K>(s1y, m), m.q);
+                r2x = add_mod(r2x, reduce_wide<K>(s2x, m), m.q);
+                r2y = add_mod(r2y, reduce_wide<K>(s2y, m), m.q);
+            });
         }
         // middle term is 2 x0 x1
         r1x = add_mod(r1x, r1x, m.q);
@@ -438,7 +445,7 @@ LB_D u64 tile_fold(const double ll, const double mid, const int shift, const dou
                        (__int128)__double2ll_rn(hh) * ((__int128)1 << 42);
     const bool neg = t < 0;
     const unsigned __int128 a = neg ? (unsigned __int128)(-t) : (unsigned __int128)t;
-    const u64 r = barrett128(u128d{(u64)a, (u64)(a >> 64)}, m.q, m.r0, m.r1);
+    const u64 r = reduce_wide(u128d{(u64)a, (u64)(a >> 64)}, m);
     return neg && r ? m.q - r : r;
 }
 
@@ -603,9 +610,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) krum_tile_kernel(const __grid
                     }
 #pragma unroll
                     for (int p = 0; p < NP; ++p) {
-                        s0[p] = u128d{barrett128(s0[p], m.q, m.r0, m.r1), 0};
-                        s1[p] = u128d{barrett128(s1[p], m.q, m.r0, m.r1), 0};
-                        s2[p] = u128d{barrett128(s2[p], m.q, m.r0, m.r1), 0};
+                        s0[p] = u128d{reduce_wide(s0[p], m), 0};
+                        s1[p] = u128d{reduce_wide(s1[p], m), 0};
+                        s2[p] = u128d{reduce_wide(s2[p], m), 0};
                     }
                 }
 #pragma unroll
@@ -811,12 +818,15 @@ __global__ void __launch_bounds__(kKrumThreads) mask_accumulate_kernel(const Mas
                 mac_wide(s2x, a1.x, b1.x);
                 mac_wide(s2y, a1.y, b1.y);
             }
-            r0x = add_mod(r0x, barrett128(s0x, m.q, m.r0, m.r1), m.q);
-            r0y = add_mod(r0y, barrett128(s0y, m.q, m.r0, m.r1), m.q);
-            r1x = add_mod(r1x, barrett128(s1x, m.q, m.r0, m.r1), m.q);
-            r1y = add_mod(r1y, barrett128(s1y, m.q, m.r0, m.r1), m.q);
-            r2x = add_mod(r2x, barrett128(s2x, m.q, m.r0, m.r1), m.q);
-            r2y = add_mod(r2y, barrett128(s2y, m.q, m.r0, m.r1), m.q);
+            with_wide_kind(m.kind, [&](auto kind) {
+                constexpr uint32_t K = decltype(kind)::value;
+                r0x = add_mod(r0x, reduce_wide<K>(s0x, m), m.q);
+                r0y = add_mod(r0y, reduce_wide<K>(s0y, m), m.q);
+                r1x = add_mod(r1x, reduce_wide<K>(s1x, m), m.q);
+                r1y = add_mod(r1y, reduce_wide<K>(s1y, m), m.q);
+                r2x = add_mod(r2x, reduce_wide<K>(s2x, m), m.q);
+                r2y = add_mod(r2y, reduce_wide<K>(s2y, m), m.q);
+            });
         }
         dst[e] = make_ulonglong2(r0x, r0y);
         dst[per_poly + e] = make_ulonglong2(r1x, r1y);
@@ -864,12 +874,15 @@ __global__ void __launch_bounds__(kPolyThreads) decrypt_kernel(const u64 *__rest
         const ModConst m = mc[(int)(i >> logN)];
         const u64 *c = ct + b * n_polys * per_poly;
         const u64 s = sk[i];
-        u64 sp = s, r = c[i];
+        // the products are added up in 128 bits and reduced once (after 32 of them at the latest)
+        u64 sp = s;
+        u128d acc = {c[i], 0};
         for (int p = 1; p < n_polys; ++p) {
-            r = add_mod(r, mul_mod(c[p * per_poly + i], sp, m.q, m.r0, m.r1), m.q);
-            sp = mul_mod(sp, s, m.q, m.r0, m.r1);
+            mac_wide(acc, c[p * per_poly + i], sp);
+            if (p + 1 < n_polys) sp = reduce_wide(mul_wide(sp, s), m);
+            if ((p & 31) == 0) acc = u128d{reduce_wide(acc, m), 0};
         }
-        pt[idx] = r;
+        pt[idx] = reduce_wide(acc, m);
     }
 }
 

@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kSampThreads) pk_combine_kernel(u64 *__restric
         u128d acc = mul_wide(a[i], s[i]);
         acc.lo += e[i];
         acc.hi += acc.lo < e[i];
-        const u64 v = barrett128(acc, m.q, m.r0, m.r1);
+        const u64 v = reduce_wide(acc, m);
         b[i] = v ? m.q - v : 0;
     }
 }
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kSampThreads) pk_combine_batch_kernel(u64 *__r
         u128d acc = mul_wide(a[i], s[i]);
         acc.lo += eb[i];
         acc.hi += acc.lo < eb[i];
-        const u64 v = barrett128(acc, m.q, m.r0, m.r1);
+        const u64 v = reduce_wide(acc, m);
         b[i] = v ? m.q - v : 0;
     }
 }
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kSampThreads) encrypt_combine_kernel(u64 *__re
             u128d acc = mul_wide(uu, pk[p * poly + k]);
             acc.lo += ee;
             acc.hi += acc.lo < ee;
-            cx[(2 * b + p) * poly + k] = barrett128(acc, m.q, m.r0, m.r1);
+            cx[(2 * b + p) * poly + k] = reduce_wide(acc, m);
         }
     }
 }
