@@ -159,6 +159,7 @@ struct FwdIn {
     const signed char *small; // the input itself as signed bytes (then src is not read)
     int n, logN;
     u64 q, r0, r1, sub_w, sub_ws, es_p;
+    const ModConst *mc;
 };
 
 LB_D u64 load_in(const FwdIn &in, const int idx)
@@ -347,6 +348,7 @@ LB_D bool fwd_row_setup(const NttK &a, const int row, FwdRow &r)
     in.n = n_in;
     in.logN = logN;
     in.q = mc.q;
+    in.mc = a.mc + tbl;
     in.r0 = mc.r0;
     in.r1 = mc.r1;
     in.src = a.src + (src_row << logN);

@@ -62,6 +62,15 @@ LB_D u64 tp_load(const u64 canonical) // a canonical residue in the form the sta
     return tp_f64(M) ? bits_of(f64_from_u52(canonical)) : canonical;
 }
 
+// a small signed value (a ternary or error coefficient) in that form
+template <int M>
+LB_D u64 tp_small(const int e, const TpPrime &p)
+{
+    if (tp_f64(M)) return bits_of(f64_from_s52((u64)(long long)e));
+    if (M == kTpNear) return p.q + (u64)(long long)e; // the stages of this class start from any word of a few q
+    return e < 0 ? p.q - (u64)(-e) : (u64)e;
+}
+
 template <int M>
 LB_D u64 tp_centre(const u64 v, const TpPrime &p) { return bits_of(f64_centre(f64_of(v), p.qd, p.qi)); }
 
@@ -87,6 +96,41 @@ LB_D u64 tp_canon(const u64 v, const TpPrime &p, const u64 r1)
     if (M == kTpNear) return csub(near_reduce(v, p.d), p.q);
     if (M == kTpLazy) return barrett64(v, p.q, r1);
     return csub(csub(csub(v, p.q << 2), p.q << 1), p.q);
+}
+
+// How the values of a row end in a fused epilogue, without a canonical form in between.  A forward transform leaves at
+// most 13.5 q (FP64, q < 2^47), 4.5 q (FP64, tight: centred here first) or 5 q + 2^32 (near 2^60).
+struct TpScale { // a fixed factor in a mode's form
+    u64 w, ws;
+};
+template <int M>
+LB_D TpScale tp_scale(const u64 w, const u64 ws, const TpPrime &p)
+{
+    if (!tp_f64(M)) return TpScale{w, ws};
+    const double wd = w > p.q / 2 ? (double)w - p.qd : (double)w;
+    return TpScale{bits_of(wd), bits_of(__dmul_rn(wd, p.qi))};
+}
+// (x - v) w + y, canonical; x, y canonical residues
+template <int M>
+LB_D u64 tp_end_scaled(const u64 v, const u64 x, const u64 y, const TpScale &w, const TpPrime &p, const u64 r1)
+{
+    if (tp_f64(M)) {
+        const double d = __dadd_rn(f64_from_u52(x), -f64_of(M == kTpF64Tight ? tp_centre<M>(v, p) : v));
+        return f64_canon(__dadd_rn(f64_mulmod(d, f64_of(w.w), f64_of(w.ws), p.qd), f64_from_u52(y)), p.qd, p.qi);
+    }
+    if (M == kTpNear) return csub(near_reduce(shoup_lazy4(x + 6 * p.q - v, w.w, w.ws, p.q) + y, p.d), p.q);
+    return add_mod(shoup_mul(sub_mod(x, tp_canon<M>(v, p, r1), p.q), w.w, w.ws, p.q), y, p.q);
+}
+// v x, canonical; x a canonical residue
+template <int M>
+LB_D u64 tp_end_product(const u64 v, const u64 x, const TpPrime &p, const u64 r0, const u64 r1)
+{
+    if (tp_f64(M)) {
+        const double w = f64_from_u52(x);
+        return f64_canon(f64_mulmod(f64_of(M == kTpF64Tight ? tp_centre<M>(v, p) : v), w, __dmul_rn(w, p.qi), p.qd), p.qd, p.qi);
+    }
+    if (M == kTpNear) return csub(near_fold(mul_wide(v, x), p.d), p.q);
+    return barrett128(mul_wide(tp_canon<M>(v, p, r1), x), p.q, r0, r1);
 }
 
 // S forward stages on canonical or settled values; tw(u, b): twiddle of block b at stage u

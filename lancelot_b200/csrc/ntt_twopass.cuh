@@ -43,71 +43,140 @@ LB_D void grid_wait()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// the transform's input at column-kernel positions j + (k << LOGST), k < V (see FwdIn)
-template <int V, int LOGST, bool PLAIN>
-LB_D void col_load(u64 (&v)[V], const FwdIn &in, const int j)
+// Sums of products of 60-bit words without carries: operands in halves of 30 bits, three products per term
+// (x0 y0, x1 y1, and (x0 - x1)(y0 - y1) for the mixed ones), and eight terms fit the 64-bit sums.
+struct Mac30 {
+    u64 ll, hh, df;
+};
+LB_D void mac30(Mac30 &s, const u64 x, const uint32_t yl, const uint32_t yh, const int yd)
+{
+    const uint32_t xl = (uint32_t)x & 0x3FFFFFFFu, xh = (uint32_t)(x >> 30);
+    s.ll += (u64)xl * yl;
+    s.hh += (u64)xh * yh;
+    s.df += (u64)((long long)((int)xl - (int)xh) * yd);
+}
+LB_D u128 mac30_sum(const Mac30 &s) // the mixed products sum to at most 16 (2^30 - 1)^2 < 2^64
+{
+    return (u128)s.ll + ((u128)(s.ll + s.hh - s.df) << 30) + ((u128)s.hh << 60);
+}
+
+// The transform's input at column-kernel positions j + (k << LOGST), k < V (see FwdIn), in the form the stages take.  FP64
+// values start at up to 1.5 q (a folded conversion and the plaintext's product), words near 2^60 at up to 2 q: each
+// stage adds 0.75 q (4 q), which keeps four stages within 4.5 q (within 16 q, see tp_fwd), and all sixteen of a prime
+// below 2^47 within 13.5 q.
+template <int V, int LOGST, int THREADS, bool PLAIN, int M>
+LB_D void col_load(u64 (&v)[V], const FwdIn &in, const TpPrime &p, const int j, u64 *own)
 {
     const u64 q = in.q;
     if (PLAIN || (in.n == 0 && in.sub == nullptr && in.small == nullptr)) {
 #pragma unroll
         for (int k = 0; k < V; ++k) v[k] = in.src[j + (k << LOGST)];
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = tp_load<M>(v[k]);
         return;
     }
+    const ModConst &m = *in.mc;
+    const bool folds = tp_f64(M) && m.kind == kWideF64;
     if (in.small) {
         // the small polynomial of an encryption as signed bytes, the same for every prime
         int ev[V];
 #pragma unroll
         for (int k = 0; k < V; ++k) ev[k] = in.small[j + (k << LOGST)];
 #pragma unroll
-        for (int k = 0; k < V; ++k) v[k] = ev[k] < 0 ? q - (u64)(-ev[k]) : (u64)ev[k];
+        for (int k = 0; k < V; ++k) v[k] = tp_small<M>(ev[k], p);
     } else if (in.n == 1 && in.mat == nullptr) {
-        // One source row reduced into this prime (every conversion of a chain with one special prime).  The branches
-        // on the optional parts stay outside the loops so that all loads of a part are in flight together.
+        // One source row reduced into this prime (every conversion of a chain with one special prime), eight words at a
+        // time.  The branches on the optional parts stay outside the loops so that all loads of a part are in flight together.
+        const TpScale w = tp_scale<M>(in.sub_w, in.sub_ws, p);
 #pragma unroll
-        for (int k = 0; k < V; ++k) v[k] = in.src[j + (k << LOGST)];
-        if (in.es) {
-            int ev[V];
+        for (int h = 0; h < V; h += 8) {
+            u64 x[8];
 #pragma unroll
-            for (int k = 0; k < V; ++k) ev[k] = in.es[j + (k << LOGST)];
+            for (int k = 0; k < 8; ++k) x[k] = in.src[j + ((h + k) << LOGST)];
+            if (in.es) {
+                int ev[8];
 #pragma unroll
-            for (int k = 0; k < V; ++k) {
-                const u64 x = add_mod(v[k], ev[k] < 0 ? in.es_p - (u64)(-ev[k]) : (u64)ev[k], in.es_p);
-                v[k] = sub_mod(barrett64(x, q, in.r1), ev[k] < 0 ? q - (u64)(-ev[k]) : (u64)ev[k], q);
+                for (int k = 0; k < 8; ++k) ev[k] = in.es[j + ((h + k) << LOGST)];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    x[k] = add_mod(x[k], ev[k] < 0 ? in.es_p - (u64)(-ev[k]) : (u64)ev[k], in.es_p);
+                    if (folds) x[k] = bits_of(f64_from_s52(f64_fold64(x[k], m) - (u64)(long long)ev[k]));
+                    else if (M == kTpNear) x[k] += q - (u64)(long long)ev[k];
+                    else x[k] = tp_load<M>(sub_mod(barrett64(x[k], q, in.r1), ev[k] < 0 ? q - (u64)(-ev[k]) : (u64)ev[k], q));
+                }
+            } else if (folds) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) x[k] = bits_of(f64_from_s52(f64_fold64(x[k], m)));
+            } else if (M != kTpNear) { // there a word of another prime, below 2^60, is hardly more than q
+#pragma unroll
+                for (int k = 0; k < 8; ++k) x[k] = tp_load<M>(barrett64(x[k], q, in.r1));
             }
-        } else {
-#pragma unroll
-            for (int k = 0; k < V; ++k) v[k] = barrett64(v[k], q, in.r1);
-        }
-        if (in.sub) {
-#pragma unroll
-            for (int h = 0; h < V; h += 8) {
+            if (in.sub) {
                 u64 t[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) t[k] = in.sub[j + ((h + k) << LOGST)];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) v[h + k] = sub_mod(v[h + k], shoup_mul(t[k], in.sub_w, in.sub_ws, q), q);
+                for (int k = 0; k < 8; ++k) {
+                    if (tp_f64(M)) x[k] = bits_of(__dadd_rn(f64_of(x[k]), -f64_mulmod(f64_from_u52(t[k]), f64_of(w.w), f64_of(w.ws), p.qd)));
+                    else if (M == kTpNear) x[k] = near_reduce(x[k] + (q << 2) - shoup_lazy4(t[k], w.w, w.ws, q), p.d);
+                    else x[k] = sub_mod(x[k], shoup_mul(t[k], w.w, w.ws, q), q);
+                }
             }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[h + k] = x[k];
         }
     } else if (in.mat != nullptr && in.sub == nullptr) {
-        // base conversion of several source rows: four outputs share one walk over the rows, so four loads are in
-        // flight per row instead of one
+        // Base conversion of several source rows: four outputs share one walk over the rows, and the words of the next row
+        // are requested before those of this one are multiplied.  Finished outputs wait in the thread's own words of shared
+        // memory (the ones its first exchange writes): the sums and two rows of operands need the registers.
+        constexpr int STEP = V < 4 ? V : 4;
+#pragma unroll 1
+        for (int h = 0; h < V; h += STEP) {
+            const u64 *src = in.src + j + (h << LOGST);
+            u64 x[STEP];
 #pragma unroll
-        for (int h = 0; h < V; h += 4) {
-            u128d acc[4];
+            for (int k = 0; k < STEP; ++k) x[k] = src[k << LOGST];
+            u128d acc[STEP];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) acc[k] = u128d{0, 0};
-            for (int i = 0; i < in.n; ++i) {
-                const u64 m = __ldg(in.mat + i);
-                const u64 *row = in.src + ((size_t)i << in.logN) + j;
+            for (int k = 0; k < STEP; ++k) acc[k] = u128d{0, 0};
+            for (int i0 = 0; i0 < in.n; i0 += 8) {
+                Mac30 s[STEP];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) mac_wide(acc[k], row[(h + k) << LOGST], m);
+                for (int k = 0; k < STEP; ++k) s[k] = Mac30{0, 0, 0};
+                const int i1 = min(i0 + 8, in.n);
+#pragma unroll 2
+                for (int i = i0; i < i1; ++i) {
+                    u64 nx[STEP];
+                    if (i + 1 < in.n) src += (size_t)1 << in.logN;
+#pragma unroll
+                    for (int k = 0; k < STEP; ++k) nx[k] = src[k << LOGST];
+                    const u64 y = __ldg(in.mat + i);
+                    const uint32_t yl = (uint32_t)y & 0x3FFFFFFFu, yh = (uint32_t)(y >> 30);
+#pragma unroll
+                    for (int k = 0; k < STEP; ++k) mac30(s[k], x[k], yl, yh, (int)yl - (int)yh);
+#pragma unroll
+                    for (int k = 0; k < STEP; ++k) x[k] = nx[k];
+                }
+#pragma unroll
+                for (int k = 0; k < STEP; ++k) {
+                    const u128 t = ((u128)acc[k].hi << 64 | acc[k].lo) + mac30_sum(s[k]);
+                    acc[k] = u128d{(u64)t, (u64)(t >> 64)};
+                }
             }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) v[h + k] = barrett128(acc[k], q, in.r0, in.r1);
+            for (int k = 0; k < STEP; ++k) {
+                u64 r;
+                if (folds) r = bits_of(f64_fold(acc[k], m));
+                else if (M == kTpNear) r = near_fold(acc[k], p.d);
+                else r = tp_load<M>(barrett128(acc[k], q, in.r0, in.r1));
+                own[(h + k) * THREADS] = r;
+            }
         }
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = own[k * THREADS];
     } else {
 #pragma unroll
-        for (int k = 0; k < V; ++k) v[k] = load_in(in, j + (k << LOGST));
+        for (int k = 0; k < V; ++k) v[k] = tp_load<M>(load_in(in, j + (k << LOGST)));
     }
 }
 
@@ -120,9 +189,7 @@ LB_D void col_fwd_body(u64 *sm, const FwdRow &fr, u64 *mid, const int tile)
     const TpPrime p = tp_prime<M>(fr.q);
     const ulonglong2 *tw = fr.tw;
     u64 v[C::V];
-    col_load<C::V, kRowLog + C::S2, PLAIN>(v, fr.in, (t << kRowLog) + col);
-#pragma unroll
-    for (int k = 0; k < C::V; ++k) v[k] = tp_load<M>(v[k]);
+    col_load<C::V, kRowLog + C::S2, C::THREADS, PLAIN, M>(v, fr.in, p, (t << kRowLog) + col, sm + threadIdx.x);
     if constexpr (C::S1 == C::S2) {
         const ulonglong2 *tg = tw + 1;
 #pragma unroll 1
@@ -169,7 +236,7 @@ template <int A, bool PLAIN>
 __global__ void __launch_bounds__(ColShape<A>::THREADS, ColShape<A>::THREADS == 256 ? 3 : 6) ntt_fwd_col_kernel(const __grid_constant__ NttK a)
 {
     using C = ColShape<A>;
-    __shared__ __align__(16) u64 sm[C::S2 ? C::V * C::THREADS : 1];
+    __shared__ __align__(16) u64 sm[C::S2 || !PLAIN ? C::V * C::THREADS : 1];
     grid_wait();
     const int row = blockIdx.x / C::TILES, tile = blockIdx.x % C::TILES;
     FwdRow fr;
@@ -244,48 +311,47 @@ LB_D void row_fwd_body(u64 *srow, const NttK &a, const RowPlace &w, const ModCon
         tg = row_twiddles(tw, logN, w.r, t, true);
     }
     const u64 r1 = mc->r1;
+    if (PLAIN || (!a.aux && !a.mul2)) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = tp_canon<M>(v[k], p, r1);
+        for (int k = 0; k < 16; ++k) v[k] = tp_canon<M>(v[k], p, r1);
+    }
     row_transpose(v, srow, t); // back to neighbouring threads on neighbouring coefficients
     if (!PLAIN && a.aux) {
         const u64 *aux = a.aux + ((size_t)(go * a.aux_outer + gi * a.aux_group_stride + w.rr) << logN) + base;
         const u64 *add = a.add1 && gi == 1 ? a.add1 + ((size_t)(go * a.add1_outer + w.rr) << logN) + base
                          : a.add && gi < a.add_inner ? a.add + ((size_t)(go * a.add_outer + gi * a.add_group_stride + w.rr) << logN) + base
                                                      : nullptr;
-        const u64 scal = a.scal[w.rr], scal_s = a.scal_s[w.rr];
+        const TpScale scal = tp_scale<M>(a.scal[w.rr], a.scal_s[w.rr], p);
 #pragma unroll
-        for (int h = 0; h < 16; h += 8) {
-            u64 x[8], y[8];
+        for (int h = 0; h < 16; h += 4) {
+            u64 x[4], y[4];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) x[k] = aux[16 * (h + k)];
+            for (int k = 0; k < 4; ++k) x[k] = aux[16 * (h + k)];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) y[k] = 0;
             if (add) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) y[k] = add[16 * (h + k)];
+                for (int k = 0; k < 4; ++k) y[k] = add[16 * (h + k)];
             }
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[h + k] = shoup_mul(sub_mod(x[k], v[h + k], q), scal, scal_s, q);
-            if (add) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) v[h + k] = add_mod(v[h + k], y[k], q);
-            }
+            for (int k = 0; k < 4; ++k) v[h + k] = tp_end_scaled<M>(v[h + k], x[k], y[k], scal, p, r1);
         }
-    }
-    if (!PLAIN && a.mul2) {
+    } else if (!PLAIN && a.mul2) {
         const u64 *mul0 = a.mul2 + ((size_t)w.rr << logN) + base, *mul1 = mul0 + ((size_t)a.per_group << logN);
         u64 *const dst1 = dst + ((size_t)a.per_group << logN);
-        const u64 m0 = mc->r0;
+        const u64 r0 = mc->r0;
 #pragma unroll
-        for (int h = 0; h < 16; h += 8) {
-            u64 x[8], y[8];
+        for (int h = 0; h < 16; h += 4) {
+            u64 x[4], y[4];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < 4; ++k) {
                 x[k] = mul0[16 * (h + k)];
                 y[k] = mul1[16 * (h + k)];
             }
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                dst1[16 * (h + k)] = barrett128(mul_wide(v[h + k], y[k]), q, m0, r1);
-                v[h + k] = barrett128(mul_wide(v[h + k], x[k]), q, m0, r1);
+            for (int k = 0; k < 4; ++k) {
+                dst1[16 * (h + k)] = tp_end_product<M>(v[h + k], y[k], p, r0, r1);
+                v[h + k] = tp_end_product<M>(v[h + k], x[k], p, r0, r1);
             }
         }
     }
