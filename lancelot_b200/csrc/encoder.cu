@@ -471,37 +471,167 @@ __global__ void __launch_bounds__(256) compose_kernel(cplx *__restrict__ out, co
     }
 }
 
-// one forward stage over global memory (fft.cu:54-182): (x0, x1) <- (x0 + w x1, x0 - w x1)
-__global__ void __launch_bounds__(256) fft_stage_kernel(cplx *__restrict__ a, const double2 *__restrict__ roots,
-                                                        const uint32_t *__restrict__ group, const int logN, const int logn,
-                                                        const int u)
+// The same for the few limbs a decoded ciphertext has in practice (Lancelot's chain: three, and two after the rescale), with
+// every word in registers: the general kernel's arrays are indexed at run time and live in local memory.
+// 342 messages of three limbs at N = 2^16: 1003 -> 338 us.
+constexpr int kSmallLimbs = 4;
+template <int L>
+struct SmallCompose {
+    u64 radix[L][L + 1], Q[L + 1], Qhalf[L + 1];
+    u64 ginv[L], ginv_s[L], radix_mod[L][L], radix_mod_s[L][L];
+};
+template <int L>
+__global__ void __launch_bounds__(256) compose_small_kernel(cplx *__restrict__ out, const u64 *__restrict__ coef,
+                                                            const ModConst *__restrict__ mc, const __grid_constant__ SmallCompose<L> cc,
+                                                            const int logN, const int logn, const double inv_scale)
 {
-    const unsigned half = 1u << (logn - 1);
-    const int logRatio = logN + 1 - logn - 2;
-    const unsigned M = 2u << logN;
-    a += (size_t)blockIdx.y << logn;
-    for (unsigned tid = blockIdx.x * blockDim.x + threadIdx.x; tid < half; tid += gridDim.x * blockDim.x) {
-        const unsigned pairs = 1u << u;
-        const unsigned k = tid >> u, j = tid & (pairs - 1), g = 2 * k * pairs + j;
-        const unsigned rev = logn > 1 ? (__brev(k << u) >> (33 - logn)) : 0u;
-        unsigned p = group[rev];
-        p <<= (u + logRatio);
-        p &= M - 1;
-        const double2 w2 = roots[p];
-        const cplx w = {w2.x, w2.y};
-        const cplx x0 = a[g], x1 = c_mul(a[g + pairs], w);
-        a[g] = c_add(x0, x1);
-        a[g + pairs] = c_sub(x0, x1);
+    constexpr int W = L + 1;
+    const unsigned n = 1u << logn, id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= 2 * n) return;
+    coef += (((size_t)blockIdx.y * L) << logN) + ((size_t)id << (logN - 1 - logn));
+    u64 t[L], v[L], x[W];
+#pragma unroll
+    for (int r = 0; r < L; ++r) t[r] = coef[(size_t)r << logN];
+#pragma unroll
+    for (int r = 0; r < L; ++r) {
+        const u64 q = mc[r].q;
+        u64 acc = 0;
+#pragma unroll
+        for (int s = 0; s < r; ++s) acc = add_mod(acc, shoup_mul(v[s], cc.radix_mod[r][s], cc.radix_mod_s[r][s], q), q);
+        v[r] = shoup_mul(sub_mod(t[r], acc, q), cc.ginv[r], cc.ginv_s[r], q);
+    }
+#pragma unroll
+    for (int i = 0; i < W; ++i) x[i] = 0;
+#pragma unroll
+    for (int r = 0; r < L; ++r) {
+        u64 carry = 0;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+            if (i > r) { // the radix has r words and a product with it r + 1
+                x[i] += carry;
+                carry = x[i] < carry;
+            } else {
+                const u128 p = (u128)cc.radix[r][i] * v[r] + x[i] + carry;
+                x[i] = (u64)p;
+                carry = (u64)(p >> 64);
+            }
+        }
+    }
+    bool gt = false, decided = false;
+#pragma unroll
+    for (int i = W - 1; i >= 0; --i)
+        if (!decided && x[i] != cc.Qhalf[i]) { gt = x[i] > cc.Qhalf[i]; decided = true; }
+    if (gt) { // x > floor(Q/2): represent x - Q
+        u64 borrow = 0;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+            const u64 a = cc.Q[i], b = x[i];
+            const u64 d = a - b - borrow;
+            borrow = (a < b) || (a == b && borrow);
+            x[i] = d;
+        }
+    }
+    double val = 0.0, word = 1.0; // L <= 4 words: 2^256 is far inside the range of a double
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+        val = __dadd_rn(val, __dmul_rn((double)x[i], word));
+        word *= 18446744073709551616.0;
+    }
+    if (gt) val = -val;
+    val *= inv_scale;
+    cplx *o = out + (size_t)blockIdx.y * n;
+    if (id < n) o[id].x = val;
+    else o[id - n].y = val;
+}
+
+// twiddle of butterfly group k at stage u of the forward transform: the conjugate of the inverse one (fft.cu:54-182)
+LB_D cplx fft_twiddle(const double2 *__restrict__ tw, const double2 *__restrict__ roots, const uint32_t *__restrict__ group, const int logN,
+                      const int logn, const unsigned k, const int u)
+{
+    if (tw) {
+        const unsigned n = 1u << logn;
+        const double2 w = __ldg(tw + (n - (n >> u)) + k);
+        return {w.x, -w.y};
+    }
+    const unsigned rev = logn > 1 ? (__brev(k << u) >> (33 - logn)) : 0u;
+    const double2 w = roots[(group[rev] << (u + logN - 1 - logn)) & ((2u << logN) - 1)];
+    return {w.x, w.y};
+}
+
+// S consecutive forward stages (spans 2^u .. 2^(u-S+1)) on 2^S values per thread: (x0, x1) <- (x0 + w x1, x0 - w x1).
+// Bound by its trips over memory, so a transform of 32768 points takes four of them instead of one per stage and one for
+// the order: 342 messages 1024 -> 353 us.  The last pass writes natural order.  There thread t takes group bitrev(t),
+// so that neighbouring threads write neighbouring values and read whole 2^S-value rows.
+constexpr int kFftPassThreads = 128;
+template <int S>
+__global__ void __launch_bounds__(kFftPassThreads) fft_pass_kernel(const cplx *in, cplx *out, const double2 *__restrict__ tw,
+                                                                   const double2 *__restrict__ roots, const uint32_t *__restrict__ group,
+                                                                   const int logN, const int logn, const int u)
+{
+    constexpr int R = 1 << S;
+    const int ul = u - S + 1; // log2 of the smallest span
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >> (logn - S)) return;
+    in += (size_t)blockIdx.y << logn;
+    out += (size_t)blockIdx.y << logn;
+    const unsigned lo = t & ((1u << ul) - 1);
+    const unsigned hi = ul > 0 ? t >> ul : logn > S ? __brev(t) >> (32 - (logn - S)) : 0u;
+    const unsigned base = (hi << (u + 1)) + lo;
+    cplx v[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = in[base + ((unsigned)i << ul)];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const int half = 1 << (S - 1 - s);
+#pragma unroll
+        for (int b = 0; b < (1 << s); ++b) {
+            const cplx w = fft_twiddle(tw, roots, group, logN, logn, (hi << s) + b, u - s);
+#pragma unroll
+            for (int i = 0; i < half; ++i) {
+                cplx &a0 = v[b * 2 * half + i], &a1 = v[b * 2 * half + i + half];
+                const cplx x1 = c_mul(a1, w), x0 = a0;
+                a0 = c_add(x0, x1);
+                a1 = c_sub(x0, x1);
+            }
+        }
+    }
+    if (ul > 0) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) out[base + ((unsigned)i << ul)] = v[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < R; ++i) out[((__brev((unsigned)i) >> (32 - S)) << (logn - S)) + t] = v[i];
     }
 }
 
-__global__ void __launch_bounds__(256) bitrev_out_kernel(cplx *__restrict__ out, const cplx *__restrict__ in, const int logn)
+template <int S>
+static void launch_fft_pass(const Context *ctx, const cplx *in, cplx *out, int logn, int u, int batch, cudaStream_t stream)
 {
-    const unsigned n = 1u << logn;
-    out += (size_t)blockIdx.y << logn;
-    in += (size_t)blockIdx.y << logn;
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[__brev(i) >> (32 - logn)] = in[i];
+    const unsigned threads = 1u << (logn - S);
+    count_launch("fft_pass_kernel", stream);
+    fft_pass_kernel<S><<<dim3((threads + kFftPassThreads - 1) / kFftPassThreads, batch), kFftPassThreads, 0, stream>>>(
+        in, out, ctx->d_ifft_tw[logn], ctx->d_croots, ctx->d_rot_group, ctx->hp.logN, logn, u);
+}
+
+template <int L>
+static void launch_compose_small(const ComposeConst &cc, const Context *ctx, cplx *buf, const u64 *coef, int logn, int batch, double inv_scale,
+                                 cudaStream_t stream)
+{
+    SmallCompose<L> sc;
+    for (int r = 0; r < L; ++r) {
+        for (int i = 0; i <= L; ++i) sc.radix[r][i] = cc.radix[r][i];
+        for (int s = 0; s < L; ++s) {
+            sc.radix_mod[r][s] = cc.radix_mod[r][s];
+            sc.radix_mod_s[r][s] = h_shoup(cc.radix_mod[r][s], ctx->hp.q[r]);
+        }
+        sc.ginv[r] = cc.ginv[r];
+        sc.ginv_s[r] = cc.ginv_s[r];
+    }
+    for (int i = 0; i <= L; ++i) {
+        sc.Q[i] = cc.Q[i];
+        sc.Qhalf[i] = cc.Qhalf[i];
+    }
+    compose_small_kernel<L><<<dim3(((2u << logn) + 255) / 256, batch), 256, 0, stream>>>(buf, coef, ctx->d_mc, sc, ctx->hp.logN, logn, inv_scale);
 }
 
 size_t decode_workspace_bytes(const Context *ctx, int size_l, int batch)
@@ -558,16 +688,26 @@ int decode(Context *ctx, int size_l, int batch, const u64 *pt, double scale, int
     }
     const unsigned n = (unsigned)sparse_slots;
     count_launch("compose_kernel", stream);
-    compose_kernel<<<dim3((2 * n + 255) / 256, batch), 256, 0, stream>>>(buf, coef, ctx->d_mc, cc, hp.logN, logn, size_l, 1.0 / scale);
-    LB_CUDA(cudaGetLastError());
-    for (int iter = 0; iter < logn; ++iter) {
-        const int u = logn - iter - 1;
-        count_launch("fft_stage_kernel", stream);
-        fft_stage_kernel<<<dim3((n / 2 + 255) / 256, batch), 256, 0, stream>>>(buf, ctx->d_croots, ctx->d_rot_group, hp.logN, logn, u);
+    switch (size_l) {
+    case 1: launch_compose_small<1>(cc, ctx, buf, coef, logn, batch, 1.0 / scale, stream); break;
+    case 2: launch_compose_small<2>(cc, ctx, buf, coef, logn, batch, 1.0 / scale, stream); break;
+    case 3: launch_compose_small<3>(cc, ctx, buf, coef, logn, batch, 1.0 / scale, stream); break;
+    case kSmallLimbs: launch_compose_small<kSmallLimbs>(cc, ctx, buf, coef, logn, batch, 1.0 / scale, stream); break;
+    default: compose_kernel<<<dim3((2 * n + 255) / 256, batch), 256, 0, stream>>>(buf, coef, ctx->d_mc, cc, hp.logN, logn, size_l, 1.0 / scale);
     }
     LB_CUDA(cudaGetLastError());
-    count_launch("bitrev_out_kernel", stream);
-    bitrev_out_kernel<<<dim3((n + 255) / 256, batch), 256, 0, stream>>>(reinterpret_cast<cplx *>(out_complex), buf, logn);
+    // as few passes of at most four stages as possible, evenly
+    for (int u = logn - 1, left = (logn + 3) / 4; left > 0; --left) {
+        const int S = (u + left) / left;
+        cplx *dst = left == 1 ? reinterpret_cast<cplx *>(out_complex) : buf;
+        switch (S) {
+        case 4: launch_fft_pass<4>(ctx, buf, dst, logn, u, batch, stream); break;
+        case 3: launch_fft_pass<3>(ctx, buf, dst, logn, u, batch, stream); break;
+        case 2: launch_fft_pass<2>(ctx, buf, dst, logn, u, batch, stream); break;
+        default: launch_fft_pass<1>(ctx, buf, dst, logn, u, batch, stream); break;
+        }
+        u -= S;
+    }
     LB_CUDA(cudaGetLastError());
     return LB_OK;
 }
