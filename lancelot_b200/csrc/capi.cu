@@ -686,7 +686,10 @@ int lb_encode_encrypt(lb_context *h, const uint64_t *pk, const void *values, int
     const size_t pt_bytes = ((size_t)batch * Q << c->hp.logN) * 8;
     if ((rc = c->ensure_workspace(enc_bytes + pt_bytes))) return rc;
     u64 *pt = reinterpret_cast<u64 *>(reinterpret_cast<uint8_t *>(c->ws) + enc_bytes);
-    if ((rc = encode(c, Q, values, dtype, (long)value_stride, n_values, sparse_slots, batch, scale, pt, c->d_status, 1, S(stream)))) return rc;
+    // the encryption's scratch (its first rows hold N / 2 complex values per message) is free while the messages are encoded
+    if ((rc = encode(c, Q, values, dtype, (long)value_stride, n_values, sparse_slots, batch, scale, pt, c->d_status, 1, S(stream),
+                     reinterpret_cast<double *>(c->ws))))
+        return rc;
     return encrypt_asymmetric(c, pk, pt, 1, seeds, batch, ct, S(stream));
 }
 

@@ -184,7 +184,7 @@ int gen_switch_keys(Context *ctx, const u64 *sk, const u64 *targets, int n, cons
 size_t encrypt_workspace_bytes(const Context *ctx, int batch);
 // encoder (encoder.cu)
 int encode(Context *ctx, int size_l, const void *values, int dtype, long value_stride, int n_values, int sparse_slots, int batch,
-           double scale, u64 *pt, int *d_status, int skip_ntt, cudaStream_t stream);
+           double scale, u64 *pt, int *d_status, int skip_ntt, cudaStream_t stream, double *mid = nullptr);
 int decode(Context *ctx, int size_l, int batch, const u64 *pt, double scale, int sparse_slots, double *out_complex, cudaStream_t stream);
 int encrypt_asymmetric(Context *ctx, const u64 *pk, const u64 *pt, int pt_is_coeff, const uint8_t *host_seeds, int batch, u64 *ct,
                        cudaStream_t stream);

@@ -10,6 +10,8 @@
 // into the final store, instead of one global pass per stage plus a host round trip.
 #include <cooperative_groups.h>
 
+#include <utility>
+
 #include "context.h"
 
 namespace cg = cooperative_groups;
@@ -102,7 +104,19 @@ LB_D void emit_coeff(const EncK &a, u64 *pt_msg, const unsigned pos, const doubl
     // ceil(log2(av)) + 1 >= total bit count  <=>  av > 2^(total - 2)   (ckks.cu:185-191)
     if (av > a.too_large) atomicOr(a.status, 1);
     const long N = 1L << a.logN;
-    if (av < 18446744073709551616.0) {
+    if (av < 2251799813685248.0) { // 2^51: what a message at Lancelot's scale of 2^40 encodes to
+        const u64 m = u52_from_f64(av);
+        for (int l = 0; l < a.size_l; ++l) {
+            const ModConst &mc = a.mc[l];
+            u64 t;
+            if (mc.kind == kWideF64) t = f64_canon(r, mc.qd, mc.qi);
+            else {
+                t = mc.q >> 51 ? m : barrett64(m, mc.q, mc.r1);
+                if (neg && t) t = mc.q - t;
+            }
+            pt_msg[l * N + pos] = t;
+        }
+    } else if (av < 18446744073709551616.0) {
         const u64 m = (u64)av;
         for (int l = 0; l < a.size_l; ++l) {
             const ModConst mc = a.mc[l];
@@ -283,6 +297,166 @@ __global__ void __launch_bounds__(kFftThreads) encode_ifft_kernel(const EncK a)
     }
 }
 
+// ---- inverse FFT in two kernels, for 4096 slots and more where scratch for the values in between is at hand ----
+// A message is a matrix of n / 256 rows of 256 values.  The row kernel gathers the input in bit-reversed order and runs the
+// stages with spans 1 .. 128, the column kernel the rest and the rounding; a thread holds 16 values and takes four
+// stages at a time in registers, with one exchange per kernel.  The cluster kernel above walks six passes with a block or
+// cluster barrier each, eight values per thread and three blocks of eight warps per SM, and waits at those barriers:
+// 51 messages of 32768 slots 110 -> 65 us.  The price is a second trip of 16 bytes per value through L2 / HBM.
+constexpr int kRowVals = 256, kEncThreads = 128, kRowsPerBlock = 8;
+constexpr int kRowStride = kRowVals + 17; // one spare value per 16 of a row, and the rows on different banks
+
+// S stages on values AT .. AT + 2^S - 1, whose lowest position bits are the register index: stage U + s, group (g << (S - 1 - s)) + b
+template <int S, int U, int AT = 0>
+LB_D void ifft_stages(double (&re)[16], double (&im)[16], const double2 *__restrict__ tw, const unsigned n, const unsigned g)
+{
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        const double2 *t = tw + (n - (n >> (U + s))) + ((size_t)g << (S - 1 - s));
+#pragma unroll
+        for (int j = 0; j < (1 << (S - 1)); ++j) {
+            const int b = j >> s, x0 = AT + (b << (s + 1)) + (j & ((1 << s) - 1)), x1 = x0 + (1 << s);
+            const double2 w = __ldg(t + b);
+            const cplx p = {re[x0], im[x0]}, q = {re[x1], im[x1]};
+            const cplx s0 = c_add(p, q), s1 = c_mul(c_sub(p, q), cplx{w.x, w.y}, U + s < kRefIfftFirstKernelStages);
+            re[x0] = s0.x;
+            im[x0] = s0.y;
+            re[x1] = s1.x;
+            im[x1] = s1.y;
+        }
+    }
+}
+// the last S stages of a column's groups of 2^S rows, whose twiddles are those of group 0
+template <int S, int... I>
+LB_D void ifft_groups(double (&re)[16], double (&im)[16], const double2 *__restrict__ tw, const unsigned n, std::integer_sequence<int, I...>)
+{
+    (ifft_stages<S, 12, I * (1 << S)>(re, im, tw, n, 0), ...);
+}
+
+// A block takes the eight rows whose input positions are neighbours (32 bytes of floats per sector read).
+__global__ void __launch_bounds__(kEncThreads, 4) encode_row_kernel(const __grid_constant__ EncK a, cplx *__restrict__ mid)
+{
+    __shared__ __align__(16) cplx sm[kRowsPerBlock * kRowStride];
+    const unsigned n = 1u << a.logn, rows_log = a.logn - 8;
+    const long msg = blockIdx.y;
+    const unsigned first = blockIdx.x * kRowsPerBlock; // the rows' bit-reversed numbers start here
+    double re[16], im[16];
+    {
+        const unsigned h = threadIdx.x & (kRowsPerBlock - 1), t = threadIdx.x / kRowsPerBlock;
+        const unsigned low = first + h + ((__brev(t) >> 28) << rows_log); // input position of value k: bitrev4(k) n / 16 + low
+        if (a.dtype == 1) {
+            const float *f = reinterpret_cast<const float *>(a.values) + msg * a.value_stride;
+            float x[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                const unsigned idx = ((__brev((unsigned)k) >> 28) << (a.logn - 4)) + low;
+                x[k] = idx < (unsigned)a.n_values ? f[idx] : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                re[k] = (double)x[k];
+                im[k] = 0.0;
+            }
+        } else if (a.dtype == 0) {
+            const double *f = reinterpret_cast<const double *>(a.values) + msg * a.value_stride;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                const unsigned idx = ((__brev((unsigned)k) >> 28) << (a.logn - 4)) + low;
+                re[k] = idx < (unsigned)a.n_values ? f[idx] : 0.0;
+                im[k] = 0.0;
+            }
+        } else {
+            const double2 *f = reinterpret_cast<const double2 *>(a.values) + msg * a.value_stride;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                const unsigned idx = ((__brev((unsigned)k) >> 28) << (a.logn - 4)) + low;
+                const double2 x = idx < (unsigned)a.n_values ? f[idx] : make_double2(0.0, 0.0);
+                re[k] = x.x;
+                im[k] = x.y;
+            }
+        }
+        const unsigned r = __brev(first + h) >> (32 - rows_log);
+        ifft_stages<4, 0>(re, im, a.tw, n, r * 16 + t);
+        cplx *row = sm + h * kRowStride + t * 17;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) row[k] = cplx{re[k], im[k]};
+    }
+    __syncthreads();
+    const unsigned h = threadIdx.x >> 4, t = threadIdx.x & 15, r = __brev(first + h) >> (32 - rows_log);
+    const cplx *row = sm + h * kRowStride + t;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const cplx z = row[17 * k];
+        re[k] = z.x;
+        im[k] = z.y;
+    }
+    ifft_stages<4, 4>(re, im, a.tw, n, r);
+    cplx *dst = mid + ((size_t)msg << a.logn) + r * kRowVals + t;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) dst[16 * k] = cplx{re[k], im[k]};
+}
+
+// A: log2 of the rows (4 .. 7).  2^(A - 4) threads per column; the twiddles depend on the row only.
+template <int A>
+__global__ void __launch_bounds__(kEncThreads, 4) encode_col_kernel(const __grid_constant__ EncK a, const cplx *__restrict__ mid)
+{
+    constexpr int S2 = A - 4, TPC = 1 << S2, COLS = kEncThreads / TPC, G = 16 >> S2;
+    __shared__ __align__(16) cplx sm[16 * kEncThreads];
+    const unsigned n = 1u << (A + 8);
+    const long msg = blockIdx.y;
+    const int cl = threadIdx.x % COLS, t = threadIdx.x / COLS, col = blockIdx.x * COLS + cl;
+    const cplx *src = mid + ((size_t)msg << (A + 8)) + col;
+    double re[16], im[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const cplx z = src[(16 * t + k) * kRowVals];
+        re[k] = z.x;
+        im[k] = z.y;
+    }
+    ifft_stages<4, 8>(re, im, a.tw, n, t);
+    if constexpr (S2 > 0) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) sm[(16 * t + k) * COLS + cl] = cplx{re[k], im[k]};
+        __syncthreads();
+        // group i of the thread: rows t + TPC i + 16 k
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const cplx z = sm[(t + TPC * (i / TPC) + 16 * (i % TPC)) * COLS + cl];
+            re[i] = z.x;
+            im[i] = z.y;
+        }
+        ifft_groups<S2>(re, im, a.tw, n, std::make_integer_sequence<int, G>());
+        __syncthreads();
+    }
+    u64 *pt_msg = a.pt + ((msg * a.size_l) << a.logN);
+    const int ratio_log = a.logN - 1 - a.logn;
+    // the rounding is long: one copy of it, fed from the thread's own words of shared memory
+#pragma unroll
+    for (int i = 0; i < 16; ++i) sm[i * kEncThreads + threadIdx.x] = cplx{re[i], im[i]};
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i) {
+        const int row = S2 > 0 ? t + TPC * (i / TPC) + 16 * (i % TPC) : i;
+        const unsigned e = (unsigned)(row * kRowVals + col);
+        cplx z = sm[i * kEncThreads + threadIdx.x];
+        if (a.fix != 0.0) {
+            z.x = __dmul_rn(z.x, a.fix);
+            z.y = __dmul_rn(z.y, a.fix);
+        }
+        emit_coeff(a, pt_msg, e << ratio_log, z.x);
+        emit_coeff(a, pt_msg, (e + n) << ratio_log, z.y);
+    }
+}
+
+template <int A>
+static void launch_encode_two(const EncK &k, int batch, cplx *mid, cudaStream_t stream)
+{
+    constexpr int COLS = kEncThreads >> (A - 4);
+    count_launch("encode_row_kernel", stream);
+    encode_row_kernel<<<dim3((1u << A) / kRowsPerBlock, (unsigned)batch), kEncThreads, 0, stream>>>(k, mid);
+    count_launch("encode_col_kernel", stream);
+    encode_col_kernel<A><<<dim3(kRowVals / COLS, (unsigned)batch), kEncThreads, 0, stream>>>(k, mid);
+}
+
 static int plan(int logn_loc, unsigned char *S)
 {
     // first pass (contiguous, gathers the input) at radix 8 when possible, then radix 8 / 4
@@ -323,8 +497,9 @@ static int launch_encode(const EncK &k, int batch, size_t smem, cudaStream_t str
 }
 
 // values -> plaintexts [batch][size_l][N] in NTT form
+// mid: scratch for batch * sparse_slots complex values, or nullptr
 int encode(Context *ctx, int size_l, const void *values, int dtype, long value_stride, int n_values, int sparse_slots, int batch,
-           double scale, u64 *pt, int *d_status, int skip_ntt, cudaStream_t stream)
+           double scale, u64 *pt, int *d_status, int skip_ntt, cudaStream_t stream, double *mid)
 {
     const HostParams &hp = ctx->hp;
     int logn = 0;
@@ -382,13 +557,24 @@ int encode(Context *ctx, int size_l, const void *values, int dtype, long value_s
     k.npass = plan(logn_loc, k.S);
     const size_t n_loc = size_t(1) << logn_loc;
     const size_t smem = (n_loc + (n_loc >> 4) + 2) * sizeof(cplx);
-    int rc;
-    switch (logc) {
-    case 0: rc = launch_encode<0>(k, batch, smem, stream); break;
-    case 1: rc = launch_encode<1>(k, batch, smem, stream); break;
-    case 2: rc = launch_encode<2>(k, batch, smem, stream); break;
-    case 3: rc = launch_encode<3>(k, batch, smem, stream); break;
-    default: set_error("slot count above 32768 is not supported"); return LB_ERR_INVALID_ARG;
+    int rc = LB_OK;
+    if (mid && logn >= 12 && logn <= 15 && batch <= 65535) {
+        cplx *m = reinterpret_cast<cplx *>(mid);
+        switch (logn) {
+        case 12: launch_encode_two<4>(k, batch, m, stream); break;
+        case 13: launch_encode_two<5>(k, batch, m, stream); break;
+        case 14: launch_encode_two<6>(k, batch, m, stream); break;
+        default: launch_encode_two<7>(k, batch, m, stream); break;
+        }
+        LB_CUDA(cudaGetLastError());
+    } else {
+        switch (logc) {
+        case 0: rc = launch_encode<0>(k, batch, smem, stream); break;
+        case 1: rc = launch_encode<1>(k, batch, smem, stream); break;
+        case 2: rc = launch_encode<2>(k, batch, smem, stream); break;
+        case 3: rc = launch_encode<3>(k, batch, smem, stream); break;
+        default: set_error("slot count above 32768 is not supported"); return LB_ERR_INVALID_ARG;
+        }
     }
     if (rc) return rc;
     if (skip_ntt) return LB_OK; // coefficient form, for an encryption that folds the plaintext in
