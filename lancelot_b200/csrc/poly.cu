@@ -786,51 +786,75 @@ int krum_accumulate_tile(Context *ctx, int size_l, int n_chunks, int n_a, const 
 constexpr int kMaxMaskClients = 64;
 
 struct MaskArgs {
-    const ulonglong2 *ct[kMaxMaskClients]; // client k, chunk c at ct[k] + c * chunk_stride
+    const u64 *ct[kMaxMaskClients]; // client k, chunk c at ct[k] + c * chunk_stride
     int n_clients;
 };
 
-__global__ void __launch_bounds__(kKrumThreads) mask_accumulate_kernel(const MaskArgs args, const ulonglong2 *__restrict__ masks,
-                                                                       ulonglong2 *__restrict__ out, const ModConst *__restrict__ mc,
-                                                                       const int log_half_n, const long per_poly,
-                                                                       const long chunk_stride)
+// A thread owns one coefficient of two consecutive chunks.  The mask words it loads serve both: with one chunk per
+// thread the masks, re-read from L2 for every chunk, were half of the words on the way to the SMs, and the kernel ran at
+// 0.55 of the copy rate.  The middle term takes one product per client, (a0 + a1)(b0 + b1) minus the outer two
+// at the end of a window (words below 2^61, so 32 products stay below 2^127).  Four clients unrolled and six blocks
+// per SM keep enough loads in flight; four chunks per thread lost to the registers of their 128-bit sums.
+// Aggregation of 20 clients x 342 chunks 7.99 -> 7.03 ms, the kernel itself 4.67 ms (4.9 TB/s).
+constexpr int kMaskChunks = 2;
+
+__global__ void __launch_bounds__(kKrumThreads, 6) mask_accumulate_kernel(const __grid_constant__ MaskArgs args, const u64 *__restrict__ masks,
+                                                                       u64 *__restrict__ out, const ModConst *__restrict__ mc,
+                                                                       const int logn, const long per_poly, const long chunk_stride,
+                                                                       const int n_chunks)
 {
-    const long c = blockIdx.y;
-    ulonglong2 *dst = out + c * 3 * per_poly;
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < per_poly; e += (long)gridDim.x * blockDim.x) {
-        const ModConst m = mc[(int)(e >> log_half_n)];
-        u64 r0x = 0, r0y = 0, r1x = 0, r1y = 0, r2x = 0, r2y = 0;
-        for (int k0 = 0; k0 < args.n_clients; k0 += 32) {
-            const int k1 = min(k0 + 32, args.n_clients);
-            u128d s0x = {0, 0}, s0y = {0, 0}, s1x = {0, 0}, s1y = {0, 0}, s2x = {0, 0}, s2y = {0, 0};
-#pragma unroll 2
-            for (int k = k0; k < k1; ++k) {
-                const ulonglong2 *a = args.ct[k] + c * chunk_stride;
-                const ulonglong2 *b = masks + (long)k * 2 * per_poly;
-                const ulonglong2 a0 = __ldcs(a + e), a1 = __ldcs(a + per_poly + e);
-                const ulonglong2 b0 = b[e], b1 = b[per_poly + e];
-                mac_wide(s0x, a0.x, b0.x);
-                mac_wide(s0y, a0.y, b0.y);
-                mac_wide(s1x, a0.x, b1.x);
-                mac_wide(s1x, a1.x, b0.x);
-                mac_wide(s1y, a0.y, b1.y);
-                mac_wide(s1y, a1.y, b0.y);
-                mac_wide(s2x, a1.x, b1.x);
-                mac_wide(s2y, a1.y, b1.y);
+    const long c0 = (long)blockIdx.y * kMaskChunks, e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= per_poly) return;
+    // chunks past the end read the last one and store nothing
+    long at[kMaskChunks];
+#pragma unroll
+    for (int c = 0; c < kMaskChunks; ++c) at[c] = min(c0 + c, (long)n_chunks - 1) * chunk_stride + e;
+    const ModConst m = mc[(int)(e >> logn)];
+    u64 r0[kMaskChunks], r1[kMaskChunks], r2[kMaskChunks];
+#pragma unroll
+    for (int c = 0; c < kMaskChunks; ++c) r0[c] = r1[c] = r2[c] = 0;
+    for (int k0 = 0; k0 < args.n_clients; k0 += 32) {
+        const int k1 = min(k0 + 32, args.n_clients);
+        u128d s0[kMaskChunks], s1[kMaskChunks], s2[kMaskChunks];
+#pragma unroll
+        for (int c = 0; c < kMaskChunks; ++c) s0[c] = s1[c] = s2[c] = u128d{0, 0};
+#pragma unroll 4
+        for (int k = k0; k < k1; ++k) {
+            const u64 *a = args.ct[k];
+            const u64 *b = masks + (long)k * 2 * per_poly + e;
+            const u64 b0 = b[0], b1 = b[per_poly], bs = b0 + b1;
+            u64 a0[kMaskChunks], a1[kMaskChunks];
+#pragma unroll
+            for (int c = 0; c < kMaskChunks; ++c) {
+                a0[c] = __ldcs(a + at[c]);
+                a1[c] = __ldcs(a + at[c] + per_poly);
             }
-            with_wide_kind(m.kind, [&](auto kind) {
-                constexpr uint32_t K = decltype(kind)::value;
-                r0x = add_mod(r0x, reduce_wide<K>(s0x, m), m.q);
-                r0y = add_mod(r0y, reduce_wide<K>(s0y, m), m.q);
-                r1x = add_mod(r1x, reduce_wide<K>(s1x, m), m.q);
-                r1y = add_mod(r1y, reduce_wide<K>(s1y, m), m.q);
-                r2x = add_mod(r2x, reduce_wide<K>(s2x, m), m.q);
-                r2y = add_mod(r2y, reduce_wide<K>(s2y, m), m.q);
-            });
+#pragma unroll
+            for (int c = 0; c < kMaskChunks; ++c) {
+                mac_wide(s0[c], a0[c], b0);
+                mac_wide(s1[c], a0[c] + a1[c], bs);
+                mac_wide(s2[c], a1[c], b1);
+            }
         }
-        dst[e] = make_ulonglong2(r0x, r0y);
-        dst[per_poly + e] = make_ulonglong2(r1x, r1y);
-        dst[2 * per_poly + e] = make_ulonglong2(r2x, r2y);
+        with_wide_kind(m.kind, [&](auto kind) {
+            constexpr uint32_t K = decltype(kind)::value;
+#pragma unroll
+            for (int c = 0; c < kMaskChunks; ++c) {
+                const u128 mid = ((u128)s1[c].hi << 64 | s1[c].lo) - ((u128)s0[c].hi << 64 | s0[c].lo) - ((u128)s2[c].hi << 64 | s2[c].lo);
+                r0[c] = add_mod(r0[c], reduce_wide<K>(s0[c], m), m.q);
+                r1[c] = add_mod(r1[c], reduce_wide<K>(u128d{(u64)mid, (u64)(mid >> 64)}, m), m.q);
+                r2[c] = add_mod(r2[c], reduce_wide<K>(s2[c], m), m.q);
+            }
+        });
+    }
+#pragma unroll
+    for (int c = 0; c < kMaskChunks; ++c) {
+        if (c0 + c < n_chunks) {
+            u64 *dst = out + (c0 + c) * 3 * per_poly + e;
+            dst[0] = r0[c];
+            dst[per_poly] = r1[c];
+            dst[2 * per_poly] = r2[c];
+        }
     }
 }
 
@@ -841,15 +865,13 @@ int mask_accumulate(Context *ctx, int size_l, int n_clients, int n_chunks, const
     if (n_chunks <= 0) return LB_OK;
     MaskArgs args;
     args.n_clients = n_clients;
-    for (int k = 0; k < n_clients; ++k) args.ct[k] = reinterpret_cast<const ulonglong2 *>(client_cts[k]);
-    const int log_half_n = ctx->hp.logN - 1;
-    const long per_poly = (long)size_l << log_half_n;
-    long blocks = (per_poly + kKrumThreads - 1) / kKrumThreads;
+    for (int k = 0; k < n_clients; ++k) args.ct[k] = client_cts[k];
+    const long per_poly = (long)size_l << ctx->hp.logN;
+    const long blocks = (per_poly + kKrumThreads - 1) / kKrumThreads;
     // every client's ciphertext read once, one size-3 sum per chunk written
     count_launch("mask_accumulate_kernel", stream, 8.0 * (size_l << ctx->hp.logN) * n_chunks * (2.0 * n_clients + 3.0));
-    mask_accumulate_kernel<<<dim3((unsigned)blocks, (unsigned)n_chunks), kKrumThreads, 0, stream>>>(
-        args, reinterpret_cast<const ulonglong2 *>(masks), reinterpret_cast<ulonglong2 *>(out), ctx->d_mc, log_half_n, per_poly,
-        chunk_stride / 2);
+    mask_accumulate_kernel<<<dim3((unsigned)blocks, (unsigned)((n_chunks + kMaskChunks - 1) / kMaskChunks)), kKrumThreads, 0, stream>>>(
+        args, masks, out, ctx->d_mc, ctx->hp.logN, per_poly, chunk_stride, n_chunks);
     LB_CUDA(cudaGetLastError());
     return LB_OK;
 }
