@@ -654,11 +654,11 @@ int lb_gen_galois_keys(lb_context *h, const uint64_t *sk, int n_keys, const int 
     const size_t poly = (size_t)c->hp.size_QP << c->hp.logN;
     uint32_t *ds;
     u64 *scratch;
-    // scratch: the rotated secret keys [n][QP][N], then one error polynomial per key and digit
-    if ((rc = stage_seeds(c, seeds, 2 * dnum * n_keys, &ds, &scratch, poly * (size_t)n_keys * (1 + dnum), S(stream)))) return rc;
+    // scratch: the rotated secret keys [n][QP][N], then one error polynomial per key and digit, then the same as signed bytes
+    const size_t errors8 = ((size_t)n_keys * dnum * c->hp.N + 7) / 8;
+    if ((rc = stage_seeds(c, seeds, 2 * dnum * n_keys, &ds, &scratch, poly * (size_t)n_keys * (1 + dnum) + errors8, S(stream)))) return rc;
     u64 *targets = scratch, *errors = scratch + poly * n_keys;
-    for (int k = 0; k < n_keys; ++k)
-        if ((rc = poly_galois(c, elt_indices[k], c->hp.size_QP, sk, targets + poly * k, S(stream)))) return rc;
+    if ((rc = poly_galois_many(c, elt_indices, n_keys, c->hp.size_QP, sk, targets, S(stream)))) return rc;
     return gen_switch_keys(c, sk, targets, n_keys, ds, out, errors, S(stream));
 }
 

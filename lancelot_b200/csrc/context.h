@@ -136,6 +136,8 @@ int poly_binary(Context *ctx, int op, int size_l, long rows, const u64 *a, const
 int poly_tensor(Context *ctx, int size_l, int batch, const u64 *a, const u64 *b, u64 *out, cudaStream_t stream);
 // dst[i] = src[perm[i]] for `rows` limbs
 int poly_galois(Context *ctx, int elt_idx, long rows, const u64 *src, u64 *dst, cudaStream_t stream);
+// dst[k] = the image of `rows` limbs under automorphism elt_idx[k], k < n
+int poly_galois_many(Context *ctx, const int *elt_idx, int n, long rows, const u64 *src, u64 *dst, cudaStream_t stream);
 // the same for ciphertexts [batch][2][L][N], with the first polynomial of each added to its own image
 int poly_galois_plus_c0(Context *ctx, int elt_idx, int L, int batch, const u64 *src, u64 *dst, cudaStream_t stream);
 int poly_sum_groups(Context *ctx, int size_l, long n_rows, int n_groups, const int *h_offsets, const int *h_indices, const u64 *in,

@@ -136,6 +136,26 @@ __global__ void __launch_bounds__(kPolyThreads) galois_kernel(const u64 *__restr
     }
 }
 
+// The images of one polynomial under several automorphisms, dst [n][rows][N]: key generation rotates the secret key for every
+// Galois key, and one launch per key spent more time between the launches than in them (26 keys at N = 2^16, with the errors kept
+// as bytes: session set-up 1113 -> 1027 us).
+constexpr int kGaloisBatch = 64;
+struct GaloisList {
+    int elt[kGaloisBatch];
+};
+__global__ void __launch_bounds__(kPolyThreads) galois_batch_kernel(const u64 *__restrict__ src, u64 *__restrict__ dst,
+                                                                    const uint32_t *__restrict__ perm, const __grid_constant__ GaloisList list,
+                                                                    const int logN, const long total)
+{
+    const long n_mask = (1L << logN) - 1;
+    perm += (size_t)list.elt[blockIdx.y] << logN;
+    dst += blockIdx.y * total;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+        const long row = i >> logN;
+        dst[i] = src[(row << logN) + perm[i & n_mask]];
+    }
+}
+
 // ciphertexts [batch][2][L][N]: dst = image of src under the automorphism, the first polynomial plus itself
 __global__ void __launch_bounds__(kPolyThreads) galois_plus_c0_kernel(const u64 *__restrict__ src, u64 *__restrict__ dst,
                                                                       const uint32_t *__restrict__ perm, const ModConst *__restrict__ mc,
@@ -204,6 +224,27 @@ int poly_galois(Context *ctx, int elt_idx, long rows, const u64 *src, u64 *dst, 
     galois_kernel<<<grid_for(ctx, total, kPolyThreads), kPolyThreads, 0, stream>>>(
         src, dst, ctx->d_perm + ((size_t)elt_idx << ctx->hp.logN), ctx->hp.logN, total);
     LB_CUDA(cudaGetLastError());
+    return LB_OK;
+}
+
+int poly_galois_many(Context *ctx, const int *elt_idx, int n, long rows, const u64 *src, u64 *dst, cudaStream_t stream)
+{
+    const long total = rows << ctx->hp.logN;
+    for (int k0 = 0; k0 < n; k0 += kGaloisBatch) {
+        const int nb = n - k0 < kGaloisBatch ? n - k0 : kGaloisBatch;
+        GaloisList list = {};
+        for (int k = 0; k < nb; ++k) {
+            if (elt_idx[k0 + k] < 0 || elt_idx[k0 + k] >= (int)ctx->hp.galois_elts.size()) {
+                set_error("Galois key not present");
+                return LB_ERR_LOGIC;
+            }
+            list.elt[k] = elt_idx[k0 + k];
+        }
+        count_launch("galois_kernel", stream);
+        galois_batch_kernel<<<dim3((unsigned)grid_for(ctx, total, kPolyThreads), (unsigned)nb), kPolyThreads, 0, stream>>>(
+            src, dst + k0 * total, ctx->d_perm, list, ctx->hp.logN, total);
+        LB_CUDA(cudaGetLastError());
+    }
     return LB_OK;
 }
 

@@ -256,7 +256,8 @@ __global__ void __launch_bounds__(kSampThreads) ksk_add_batch_kernel(u64 *__rest
 
 // n switch keys at once: the streams, and so the keys, are those of n calls of gen_switch_key with seeds
 // d_seeds + k * 32 * dnum, but every step is one launch over all keys and digits instead of one per key and digit.
-// targets: [n][QP][N]; out: [n][dnum][2][QP][N]; scratch: n * dnum polynomials.
+// targets: [n][QP][N]; out: [n][dnum][2][QP][N]; scratch: n * dnum polynomials [QP][N] and as many of N bytes behind them.
+// The errors stay signed bytes between sampler and transform, which reads a byte per coefficient and prime instead of a word.
 int gen_switch_keys(Context *ctx, const u64 *sk, const u64 *targets, int n, const uint32_t *d_seeds, u64 *out, u64 *scratch,
                     cudaStream_t stream)
 {
@@ -267,9 +268,13 @@ int gen_switch_keys(Context *ctx, const u64 *sk, const u64 *targets, int n, cons
     if (pairs == 0) return LB_OK;
     if (pairs > 65535) { set_error("too many switch keys in one call"); return LB_ERR_INVALID_ARG; }
     int rc;
-    if ((rc = sample_small(ctx, 1, d_seeds, 32, pairs, hp.size_Q, hp.size_P, scratch, stream))) return rc;
+    signed char *errors = reinterpret_cast<signed char *>(scratch + (size_t)pairs * poly);
+    const long n_small = (long)pairs << hp.logN;
+    count_launch("sample_small_i8_kernel", stream, (double)n_small);
+    sample_small_i8_kernel<<<grid_for(ctx, n_small), kSampThreads, 0, stream>>>(errors, d_seeds, 32, 1, hp.logN, n_small);
+    LB_CUDA(cudaGetLastError());
     NttJob j;
-    j.src = scratch;
+    j.small = errors;
     j.dst = scratch;
     j.n_groups = pairs;
     j.per_group = hp.size_QP;
