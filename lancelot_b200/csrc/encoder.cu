@@ -96,6 +96,9 @@ LB_D cplx ifft_twiddle(const EncK &a, const unsigned k, const int u)
 }
 
 // round, reduce into every prime, and store coefficient `pos` of the plaintext (rns_base.cu:121-156)
+// QUOT_F64: coefficients below 2^51 take their quotients on the FP64 pipe.  Not in the cluster kernels: their unrolled copies
+// of the longer code cost a product chain at N = 2^13 30 us.
+template <bool QUOT_F64>
 LB_D void emit_coeff(const EncK &a, u64 *pt_msg, const unsigned pos, const double value)
 {
     const double r = round(value);
@@ -104,7 +107,7 @@ LB_D void emit_coeff(const EncK &a, u64 *pt_msg, const unsigned pos, const doubl
     // ceil(log2(av)) + 1 >= total bit count  <=>  av > 2^(total - 2)   (ckks.cu:185-191)
     if (av > a.too_large) atomicOr(a.status, 1);
     const long N = 1L << a.logN;
-    if (av < 2251799813685248.0) { // 2^51: what a message at Lancelot's scale of 2^40 encodes to
+    if (QUOT_F64 && av < 2251799813685248.0) { // 2^51: what a message at Lancelot's scale of 2^40 encodes to
         const u64 m = u52_from_f64(av);
         for (int l = 0; l < a.size_l; ++l) {
             const ModConst &mc = a.mc[l];
@@ -201,8 +204,8 @@ LB_D void ifft_pass(cplx *sm, const EncK &a, const long msg, const bool first, c
                     z.x = __dmul_rn(z.x, a.fix);
                     z.y = __dmul_rn(z.y, a.fix);
                 }
-                emit_coeff(a, pt_msg, e << ratio_log, z.x);
-                emit_coeff(a, pt_msg, (e + n) << ratio_log, z.y);
+                emit_coeff<false>(a, pt_msg, e << ratio_log, z.x);
+                emit_coeff<false>(a, pt_msg, (e + n) << ratio_log, z.y);
             }
         } else {
 #pragma unroll
@@ -289,8 +292,8 @@ __global__ void __launch_bounds__(kFftThreads) encode_ifft_kernel(const EncK a)
                     z.x = __dmul_rn(z.x, a.fix);
                     z.y = __dmul_rn(z.y, a.fix);
                 }
-                emit_coeff(a, pt_msg, e << ratio_log, z.x);
-                emit_coeff(a, pt_msg, (e + n) << ratio_log, z.y);
+                emit_coeff<false>(a, pt_msg, e << ratio_log, z.x);
+                emit_coeff<false>(a, pt_msg, (e + n) << ratio_log, z.y);
             }
         }
         cluster.sync();
@@ -442,8 +445,8 @@ __global__ void __launch_bounds__(kEncThreads, 4) encode_col_kernel(const __grid
             z.x = __dmul_rn(z.x, a.fix);
             z.y = __dmul_rn(z.y, a.fix);
         }
-        emit_coeff(a, pt_msg, e << ratio_log, z.x);
-        emit_coeff(a, pt_msg, (e + n) << ratio_log, z.y);
+        emit_coeff<true>(a, pt_msg, e << ratio_log, z.x);
+        emit_coeff<true>(a, pt_msg, (e + n) << ratio_log, z.y);
     }
 }
 
