@@ -120,6 +120,7 @@ LB_API int lb_galois_permute(lb_context *ctx, int elt_index, int n_limbs, const 
 
 LB_API int lb_modup(lb_context *ctx, int size_l, const uint64_t *cks, uint64_t *digits, void *stream);
 LB_API int lb_keyswitch_inner_product(lb_context *ctx, int size_l, const uint64_t *digits, const uint64_t *evk, uint64_t *cx, void *stream);
+/* cx[size_l + size_P][N] -> out[size_l][N]; out may be cx */
 LB_API int lb_moddown(lb_context *ctx, int size_l, const uint64_t *cx, uint64_t *out, void *stream);
 /* switch_key_inplace: ct[2][size_l][N] += KS(cks) */
 LB_API int lb_keyswitch(lb_context *ctx, int size_l, uint64_t *ct, const uint64_t *cks, const uint64_t *evk, void *stream);

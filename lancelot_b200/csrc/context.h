@@ -118,12 +118,15 @@ struct NttJob {
     // public key); group g stores NTT(x) * mul2[0] at dst rows (go * dst_outer + rr) and NTT(x) * mul2[1] per_group rows
     // further on, so dst_outer = 2 * per_group lays the products out as [group][2][per_group][N]
     const u64 *mul2 = nullptr;
-    // Rows the forward transform may keep its values in between its two kernels, one per row of the job, for jobs whose
-    // aux / add rows alias dst; nullptr: the dst rows themselves
+    // Rows the forward transform keeps its values in between its two kernels, one per row of the job; nullptr: the dst rows
+    // themselves.  Needed wherever dst may share memory with the aux / add rows, which only the second kernel reads
     u64 *mid = nullptr;
     // Inverse epilogue: closing constants per row replaced by fold[rr][4]
     const u64 *fold = nullptr;
 };
+
+// true: the two ranges of words share memory
+inline bool overlaps(const u64 *a, size_t na, const u64 *b, size_t nb) { return a < b + nb && b < a + na; }
 
 int ntt_forward(Context *ctx, const NttJob &job, cudaStream_t stream);
 int ntt_inverse(Context *ctx, const NttJob &job, cudaStream_t stream);

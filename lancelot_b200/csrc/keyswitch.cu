@@ -366,7 +366,9 @@ int moddown(Context *ctx, int L, const u64 *cx, u64 *out, cudaStream_t stream)
     if (rc) return rc;
     KsWs w;
     if ((rc = get_ws(ctx, L, 1, w))) return rc;
-    return moddown_into(ctx, L, 1, 1, cx, w.pc, out, Placement{L, L}, nullptr, Placement{0, 0}, 0, nullptr, stream);
+    const size_t N = ctx->hp.N;
+    u64 *const mid = overlaps(out, L * N, cx, (L + ctx->hp.size_P) * N) ? w.digits : nullptr;
+    return moddown_into(ctx, L, 1, 1, cx, w.pc, out, Placement{L, L}, nullptr, Placement{0, 0}, 0, mid, stream);
 }
 
 // out(b, p) = (p < add_inner ? add(b, p) : 0) + moddown(<modup(cks_b), evk>)_p for a batch of ciphertexts
