@@ -422,7 +422,10 @@ int rescale(Context *ctx, int L, int batch, int ppc, const u64 *in, long in_oute
 {
     if (L < 2 || L > ctx->hp.size_Q) { set_error("cannot rescale: no next level"); return LB_ERR_INVALID_ARG; }
     const int n_polys = batch * ppc;
-    int rc = ctx->ensure_workspace((size_t)n_polys * ctx->hp.N * 8);
+    if (n_polys < 1) return LB_OK;
+    const size_t N = ctx->hp.N, out_words = (size_t)n_polys * (L - 1) * N;
+    const bool in_place = overlaps(out, out_words, in, ((size_t)(batch - 1) * in_outer + (size_t)ppc * L) * N);
+    int rc = ctx->ensure_workspace((n_polys * N + (in_place ? out_words : 0)) * 8);
     if (rc) return rc;
     u64 *last = reinterpret_cast<u64 *>(ctx->ws);
     NttJob inv;
@@ -454,6 +457,7 @@ int rescale(Context *ctx, int L, int batch, int ppc, const u64 *in, long in_oute
     fwd.aux_outer = in_outer;
     fwd.scal = dl.qlast_inv;
     fwd.scal_s = dl.qlast_inv_s;
+    fwd.mid = in_place ? last + n_polys * N : nullptr;
     return ntt_forward(ctx, fwd, stream);
 }
 

@@ -37,3 +37,20 @@ def test_mod_down(oracle_mod, logn, chain):
         check(lib.lb_moddown(ctx.h, L, p, p, ctx._stream()))
         got = cabi.to_host(d).reshape(L + P, n)
         assert np.array_equal(got[:L], want) and np.array_equal(got[L:], cx[L:])
+
+
+@pytest.mark.parametrize("logn", [11, 12, 13, 15, 16])
+@pytest.mark.parametrize("chain", CHAINS)
+@pytest.mark.parametrize("entry", ["lb_rescale"])
+def test_rescale_of_one_polynomial(oracle_mod, logn, chain, entry):
+    from lancelot_b200 import cabi
+    from lancelot_b200._lib import check, lib
+
+    o, ctx, mods, Q, _ = _setup(oracle_mod, logn, chain)
+    n, rng = 1 << logn, np.random.default_rng(logn)
+    for L in (Q, 2):
+        x = rand_rows(rng, mods[:L], n)
+        d = cabi.to_device(x[None])
+        p = C.c_void_p(d.data_ptr())
+        check(getattr(lib, entry)(ctx.h, L, 1, p, p, ctx._stream()))
+        assert np.array_equal(cabi.to_host(d).reshape(L, n)[:L - 1], o.rescale(L, x[None]).reshape(L - 1, n))
