@@ -126,7 +126,9 @@ LB_API int lb_moddown(lb_context *ctx, int size_l, const uint64_t *cx, uint64_t 
 LB_API int lb_keyswitch(lb_context *ctx, int size_l, uint64_t *ct, const uint64_t *cks, const uint64_t *evk, void *stream);
 /* relinearize_inplace (cahel-main/src/evaluate.cu:2019): ct3[3][size_l][N]; result in the first two polynomials */
 LB_API int lb_relinearize(lb_context *ctx, int size_l, uint64_t *ct3, const uint64_t *relin_key, void *stream);
-/* rescale_to_next (cahel-main/src/evaluate.cu:2059,2307; rns.cu:544): in [n_polys][size_l][N] -> out [n_polys][size_l-1][N] */
+/* rescale_to_next (cahel-main/src/evaluate.cu:2059,2307; rns.cu:544): in [n_polys][size_l][N] -> out [n_polys][size_l-1][N].
+ * A single polynomial may be rescaled in place (out == in, n_polys == 1), here and in lb_rescale_no_alloc; otherwise the
+ * two must not overlap. */
 LB_API int lb_rescale(lb_context *ctx, int size_l, int n_polys, const uint64_t *in, uint64_t *out, void *stream);
 /* rescale of the first polys_per_ct polynomials of `batch` ciphertexts that sit ct_stride words apart
  * (e.g. the two result polynomials of relinearized size-3 ciphertexts); out is dense [batch][polys_per_ct][size_l-1][N] */

@@ -88,7 +88,24 @@ int rescale_static(Context *ctx, int L, int n_polys, const u64 *in, u64 *out, cu
     fwd.aux_group_stride = L;
     fwd.scal = dl.qlast_inv;
     fwd.scal_s = dl.qlast_inv_s;
-    return ntt_forward(ctx, fwd, stream);
+    const size_t N = ctx->hp.N, room = kStaticWords / N - n_polys;
+    if (n_polys > 1 || room < 1 || !overlaps(out, (L - 1) * N, in, L * N)) return ntt_forward(ctx, fwd, stream);
+    // One polynomial in place: the rest of the array takes the rows between the transform's two kernels, so the limbs
+    // go through in groups of as many as there is room for (two at a ring degree of 65536; a ring of 131072 has none left
+    // and needs none, its transforms are one kernel).
+    fwd.mid = last + N;
+    for (int l = 0; l < L - 1; l += (int)room) {
+        const int n = L - 1 - l < (int)room ? L - 1 - l : (int)room;
+        fwd.tbl_off = l;
+        fwd.per_group = n;
+        fwd.size_l = n;
+        fwd.dst = out + l * N;
+        fwd.aux = in + l * N;
+        fwd.scal = dl.qlast_inv + l;
+        fwd.scal_s = dl.qlast_inv_s + l;
+        if ((rc = ntt_forward(ctx, fwd, stream))) return rc;
+    }
+    return LB_OK;
 }
 
 } // namespace lb

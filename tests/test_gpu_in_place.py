@@ -41,7 +41,7 @@ def test_mod_down(oracle_mod, logn, chain):
 
 @pytest.mark.parametrize("logn", [11, 12, 13, 15, 16])
 @pytest.mark.parametrize("chain", CHAINS)
-@pytest.mark.parametrize("entry", ["lb_rescale"])
+@pytest.mark.parametrize("entry", ["lb_rescale", "lb_rescale_no_alloc"])
 def test_rescale_of_one_polynomial(oracle_mod, logn, chain, entry):
     from lancelot_b200 import cabi
     from lancelot_b200._lib import check, lib
