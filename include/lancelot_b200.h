@@ -227,7 +227,8 @@ LB_API int lb_gen_switch_key(lb_context *ctx, const uint64_t *sk, const uint64_t
 LB_API int lb_gen_galois_keys(lb_context *ctx, const uint64_t *sk, int n_keys, const int *elt_indices, const uint8_t *seeds,
                        uint64_t *out, void *stream);
 /* encrypt_asymmetric (secretkey.cu:47-249) for a batch: ct[b][2][size_Q][N] = moddown(pk u + e) + (pt[b], 0).
- * seeds[b][2][64] = (ternary seed, error seed); pt may be NULL (encryption of zero). */
+ * seeds[b][2][64] = (ternary seed, error seed); pt may be NULL (encryption of zero).  With batch == 1 pt may be the first
+ * polynomial of ct; otherwise the two must not overlap. */
 LB_API int lb_encrypt_asymmetric(lb_context *ctx, const uint64_t *pk, const uint64_t *pt, const uint8_t *seeds, int batch, uint64_t *ct, void *stream);
 
 /* ---- CKKS encoder (cahel-main/src/ckks.cu:104-209,292-465) ---------------------------------- */

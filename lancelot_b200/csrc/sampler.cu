@@ -344,6 +344,8 @@ int encrypt_asymmetric(Context *ctx, const u64 *pk, const u64 *pt, int pt_is_coe
     // seeds arrive as [batch][2][64 bytes]: (ternary seed, error seed) per ciphertext
     LB_CUDA(cudaMemcpyAsync(seeds, host_seeds, (size_t)batch * 128, cudaMemcpyHostToDevice, stream));
     const bool fold_e = (P == 1); // one special prime: the error never needs its own transforms
+    // folded errors are bytes at the end of e, so that the rows before them are free once u has been transformed
+    signed char *const e8 = reinterpret_cast<signed char *>(cx) - (size_t)batch * hp.N;
     const long total = batch * poly;
     if (fold_e) {
         // u and e stay signed bytes: the transforms that consume them reduce them into their primes while loading
@@ -353,8 +355,7 @@ int encrypt_asymmetric(Context *ctx, const u64 *pk, const u64 *pt, int pt_is_coe
                                                                                    n_small);
         LB_CUDA(cudaGetLastError());
         count_launch("sample_small_i8_kernel", stream, (double)n_small);
-        sample_small_i8_kernel<<<grid_for(ctx, n_small), kSampThreads, 0, stream>>>(reinterpret_cast<signed char *>(e), seeds + 16, 32, 1,
-                                                                                   hp.logN, n_small);
+        sample_small_i8_kernel<<<grid_for(ctx, n_small), kSampThreads, 0, stream>>>(e8, seeds + 16, 32, 1, hp.logN, n_small);
         LB_CUDA(cudaGetLastError());
         // u's transform stores its products with the two key polynomials straight away: cx[b][p][QP][N] = pk[p] * NTT(u[b])
         NttJob j;
@@ -410,7 +411,7 @@ int encrypt_asymmetric(Context *ctx, const u64 *pk, const u64 *pt, int pt_is_coe
     fwd.scal_s = dl.p_inv_s;
     fwd.split = 2;
     if (fold_e) {
-        fwd.esmall = reinterpret_cast<const signed char *>(e);
+        fwd.esmall = e8;
         fwd.esmall_p = hp.q[Q];
     }
     if (pt && pt_is_coeff) {
@@ -424,6 +425,8 @@ int encrypt_asymmetric(Context *ctx, const u64 *pk, const u64 *pt, int pt_is_coe
         fwd.add_group_stride = 0;
         fwd.add_outer = Q;
         fwd.add_inner = pt ? 1 : 0;
+        // a plaintext inside its own result; 2 batch Q rows fit before the error bytes
+        if (pt && overlaps(pt, (size_t)batch * Q << hp.logN, ct, (size_t)2 * batch * Q << hp.logN)) fwd.mid = u;
     }
     return ntt_forward(ctx, fwd, stream);
 }

@@ -54,3 +54,18 @@ def test_rescale_of_one_polynomial(oracle_mod, logn, chain, entry):
         p = C.c_void_p(d.data_ptr())
         check(getattr(lib, entry)(ctx.h, L, 1, p, p, ctx._stream()))
         assert np.array_equal(cabi.to_host(d).reshape(L, n)[:L - 1], o.rescale(L, x[None]).reshape(L - 1, n))
+
+
+@pytest.mark.parametrize("logn", [11, 12, 13])
+@pytest.mark.parametrize("chain", CHAINS)
+def test_encryption_of_a_plaintext_in_its_result(oracle_mod, logn, chain):
+    from lancelot_b200 import cabi
+
+    o, ctx, mods, Q, _ = _setup(oracle_mod, logn, chain)
+    n, rng = 1 << logn, np.random.default_rng(logn)
+    pk = o.gen_pk(o.gen_sk(seeds(rng, 1)), seeds(rng, 1), seeds(rng, 1))
+    pt, s = rand_rows(rng, mods[:Q], n), seeds(rng, 2)
+    ct = ctx.empty(1, 2, Q, n)
+    ct[0, 0] = cabi.to_device(pt)
+    ctx.encrypt_asymmetric(cabi.to_device(pk), ct[0, 0], s, 1, out=ct)
+    assert np.array_equal(cabi.to_host(ct).reshape(2, Q, n), o.encrypt_asym(pk, pt, s[:64], s[64:]))
