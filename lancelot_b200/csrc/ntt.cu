@@ -741,7 +741,7 @@ static int launch(bool forward, const NttK &k, int rows, size_t smem, cudaStream
     return LB_OK;
 }
 
-// `grid` blocks of `threads`; the kernel may start while its predecessor in the stream drains (see grid_wait)
+// `grid` blocks of `threads`; the kernel is set up while its predecessor in the stream ends (see grid_wait)
 static int launch_serial(void (*kern)(const NttK), const NttK &k, long grid, int threads, cudaStream_t stream)
 {
     cudaLaunchConfig_t cfg = {};
