@@ -975,7 +975,9 @@ __global__ void __launch_bounds__(kPolyThreads) decrypt_kernel(const u64 *__rest
 {
     for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long)gridDim.x * blockDim.x) {
         const long b = idx / per_poly, i = idx - b * per_poly;
-        const ModConst m = mc[(int)(i >> logN)];
+        // the constants are read where the prime's class needs them: all of them up front, 112 bytes per element, took 86.0 us
+        // instead of 72.8 for six ciphertexts of 24 limbs (82.9 with the two-word quotient for every prime)
+        const ModConst &m = mc[(int)(i >> logN)];
         const u64 *c = ct + b * n_polys * per_poly;
         const u64 s = sk[i];
         // the products are added up in 128 bits and reduced once (after 32 of them at the latest)
