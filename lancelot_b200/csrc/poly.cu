@@ -872,47 +872,42 @@ struct MaskArgs {
     int n_clients;
 };
 
-// A thread owns one coefficient of two consecutive chunks.  The mask words it loads serve both: with one chunk per
-// thread the masks, re-read from L2 for every chunk, were half of the words on the way to the SMs, and the kernel ran at
-// 0.55 of the copy rate.  The middle term takes one product per client, (a0 + a1)(b0 + b1) minus the outer two
-// at the end of a window (words below 2^61, so 32 products stay below 2^127).  Four clients unrolled and six blocks
-// per SM keep enough loads in flight; four chunks per thread lost to the registers of their 128-bit sums.
-// Aggregation of 20 clients x 342 chunks 7.99 -> 7.03 ms, the kernel itself 4.67 ms (4.9 TB/s).
+// A thread owns one coefficient of two consecutive chunks, of the last one alone where their number is odd.  The mask words it
+// loads serve both: with one chunk per thread the masks, re-read from L2 for every chunk, were half of the words on the way to the
+// SMs, and the kernel ran at 0.55 of the copy rate.  The middle term takes one product per client, (a0 + a1)(b0 + b1) minus the
+// outer two at the end of a window (words below 2^61, so 32 products stay below 2^127).  Four clients unrolled and six blocks per
+// SM keep enough loads in flight; four chunks per thread lost to the registers of their 128-bit sums, and so did the prime's
+// constants held in registers (264 bytes spilt; they are read where the sums are reduced).  20 clients x 16 chunks of N = 2^16
+// 307.9 -> 206.3 us (4.8 TB/s), 3 clients x 3 chunks 16.5 -> 14.4; a second, idle chunk in place of the odd one took 20.5.
 constexpr int kMaskChunks = 2;
 
-__global__ void __launch_bounds__(kKrumThreads, 6) mask_accumulate_kernel(const __grid_constant__ MaskArgs args, const u64 *__restrict__ masks,
-                                                                       u64 *__restrict__ out, const ModConst *__restrict__ mc,
-                                                                       const int logn, const long per_poly, const long chunk_stride,
-                                                                       const int n_chunks)
+// C chunks from chunk c0 on, one coefficient of each
+template <int C>
+LB_D void mask_sums(const MaskArgs &args, const u64 *__restrict__ masks, u64 *__restrict__ out, const ModConst &m, const long e,
+                    const long per_poly, const long chunk_stride, const long c0)
 {
-    const long c0 = (long)blockIdx.y * kMaskChunks, e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= per_poly) return;
-    // chunks past the end read the last one and store nothing
-    long at[kMaskChunks];
+    const long at = c0 * chunk_stride + e;
+    u64 r0[C], r1[C], r2[C];
 #pragma unroll
-    for (int c = 0; c < kMaskChunks; ++c) at[c] = min(c0 + c, (long)n_chunks - 1) * chunk_stride + e;
-    const ModConst m = mc[(int)(e >> logn)];
-    u64 r0[kMaskChunks], r1[kMaskChunks], r2[kMaskChunks];
-#pragma unroll
-    for (int c = 0; c < kMaskChunks; ++c) r0[c] = r1[c] = r2[c] = 0;
+    for (int c = 0; c < C; ++c) r0[c] = r1[c] = r2[c] = 0;
     for (int k0 = 0; k0 < args.n_clients; k0 += 32) {
         const int k1 = min(k0 + 32, args.n_clients);
-        u128d s0[kMaskChunks], s1[kMaskChunks], s2[kMaskChunks];
+        u128d s0[C], s1[C], s2[C];
 #pragma unroll
-        for (int c = 0; c < kMaskChunks; ++c) s0[c] = s1[c] = s2[c] = u128d{0, 0};
+        for (int c = 0; c < C; ++c) s0[c] = s1[c] = s2[c] = u128d{0, 0};
 #pragma unroll 4
         for (int k = k0; k < k1; ++k) {
-            const u64 *a = args.ct[k];
+            const u64 *a = args.ct[k] + at;
             const u64 *b = masks + (long)k * 2 * per_poly + e;
             const u64 b0 = b[0], b1 = b[per_poly], bs = b0 + b1;
-            u64 a0[kMaskChunks], a1[kMaskChunks];
+            u64 a0[C], a1[C];
 #pragma unroll
-            for (int c = 0; c < kMaskChunks; ++c) {
-                a0[c] = __ldcs(a + at[c]);
-                a1[c] = __ldcs(a + at[c] + per_poly);
+            for (int c = 0; c < C; ++c) {
+                a0[c] = __ldcs(a + c * chunk_stride);
+                a1[c] = __ldcs(a + c * chunk_stride + per_poly);
             }
 #pragma unroll
-            for (int c = 0; c < kMaskChunks; ++c) {
+            for (int c = 0; c < C; ++c) {
                 mac_wide(s0[c], a0[c], b0);
                 mac_wide(s1[c], a0[c] + a1[c], bs);
                 mac_wide(s2[c], a1[c], b1);
@@ -921,7 +916,7 @@ __global__ void __launch_bounds__(kKrumThreads, 6) mask_accumulate_kernel(const 
         with_wide_kind(m.kind, [&](auto kind) {
             constexpr uint32_t K = decltype(kind)::value;
 #pragma unroll
-            for (int c = 0; c < kMaskChunks; ++c) {
+            for (int c = 0; c < C; ++c) {
                 const u128 mid = ((u128)s1[c].hi << 64 | s1[c].lo) - ((u128)s0[c].hi << 64 | s0[c].lo) - ((u128)s2[c].hi << 64 | s2[c].lo);
                 r0[c] = add_mod(r0[c], reduce_wide<K>(s0[c], m), m.q);
                 r1[c] = add_mod(r1[c], reduce_wide<K>(u128d{(u64)mid, (u64)(mid >> 64)}, m), m.q);
@@ -930,14 +925,24 @@ __global__ void __launch_bounds__(kKrumThreads, 6) mask_accumulate_kernel(const 
         });
     }
 #pragma unroll
-    for (int c = 0; c < kMaskChunks; ++c) {
-        if (c0 + c < n_chunks) {
-            u64 *dst = out + (c0 + c) * 3 * per_poly + e;
-            dst[0] = r0[c];
-            dst[per_poly] = r1[c];
-            dst[2 * per_poly] = r2[c];
-        }
+    for (int c = 0; c < C; ++c) {
+        u64 *dst = out + (c0 + c) * 3 * per_poly + e;
+        dst[0] = r0[c];
+        dst[per_poly] = r1[c];
+        dst[2 * per_poly] = r2[c];
     }
+}
+
+__global__ void __launch_bounds__(kKrumThreads, 6) mask_accumulate_kernel(const __grid_constant__ MaskArgs args, const u64 *__restrict__ masks,
+                                                                       u64 *__restrict__ out, const ModConst *__restrict__ mc,
+                                                                       const int logn, const long per_poly, const long chunk_stride,
+                                                                       const int n_chunks)
+{
+    const long c0 = (long)blockIdx.y * kMaskChunks, e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= per_poly) return;
+    const ModConst &m = mc[(int)(e >> logn)];
+    if (c0 + kMaskChunks <= n_chunks) mask_sums<kMaskChunks>(args, masks, out, m, e, per_poly, chunk_stride, c0);
+    else mask_sums<1>(args, masks, out, m, e, per_poly, chunk_stride, c0);
 }
 
 int mask_accumulate(Context *ctx, int size_l, int n_clients, int n_chunks, const u64 *const *client_cts, long chunk_stride,
