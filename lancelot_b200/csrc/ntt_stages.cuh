@@ -10,25 +10,26 @@
 //                word v comes back to about q by (v mod 2^60) + (v >> 60) (2^60 - q), three instructions
 //                against six of a conditional subtraction, and 64 bits hold 16 q, so the forward stages reduce
 //                half of the values once per four stages instead of a value per butterfly.
-//   integer      the remaining integer primes keep the butterflies of ntt_butterfly.cuh.
+//   integer      the remaining primes of 50 bits and more keep values in [0, 8q) with a conditional subtraction per butterfly.
+//                A class of its own for primes below 2^58, without that subtraction but with the four-multiplication product,
+//                was 1 to 4 % slower (768 limbs of 57 bits at N = 2^15 292 us against 282).
 #pragma once
 #include "ntt_butterfly.cuh"
 
 namespace lb {
 
 // butterfly kinds of the two-kernel transforms
-enum { kTpStrict = 0, kTpLazy = 1, kTpNear = 2, kTpF64Tight = 3, kTpF64 = 4 };
+enum { kTpStrict = 0, kTpNear = 1, kTpF64Tight = 2, kTpF64 = 3 };
 LB_D constexpr bool tp_f64(const int m) { return m == kTpF64 || m == kTpF64Tight; }
 
 // primes below 2^42 need no reduction inside a kernel of an inverse transform (sums of at most nine stages)
 constexpr u64 kF64InvPrimeLimit = u64(1) << 42;
 
-LB_D int tp_fwd_mode(const u64 q)
+LB_HD int tp_fwd_mode(const u64 q)
 {
     if (q < kF64PrimeLimit) return kTpF64;
     if (q < kF64TightPrimeLimit) return kTpF64Tight;
-    if ((q >> 58) == 0) return kTpLazy;
-    return kNearTop - q < kNearSpan ? kTpNear : kTpStrict;
+    return q < kNearTop && kNearTop - q < kNearSpan ? kTpNear : kTpStrict;
 }
 LB_D int tp_inv_mode(const u64 q)
 {
@@ -90,11 +91,10 @@ LB_D void tp_settle(u64 (&v)[R], const TpPrime &p)
 
 // value left by the stages -> canonical residue
 template <int M>
-LB_D u64 tp_canon(const u64 v, const TpPrime &p, const u64 r1)
+LB_D u64 tp_canon(const u64 v, const TpPrime &p)
 {
     if (tp_f64(M)) return f64_canon(f64_of(v), p.qd, p.qi);
     if (M == kTpNear) return csub(near_reduce(v, p.d), p.q);
-    if (M == kTpLazy) return barrett64(v, p.q, r1);
     return csub(csub(csub(v, p.q << 2), p.q << 1), p.q);
 }
 
@@ -112,14 +112,14 @@ LB_D TpScale tp_scale(const u64 w, const u64 ws, const TpPrime &p)
 }
 // (x - v) w + y, canonical; x, y canonical residues
 template <int M>
-LB_D u64 tp_end_scaled(const u64 v, const u64 x, const u64 y, const TpScale &w, const TpPrime &p, const u64 r1)
+LB_D u64 tp_end_scaled(const u64 v, const u64 x, const u64 y, const TpScale &w, const TpPrime &p)
 {
     if (tp_f64(M)) {
         const double d = __dadd_rn(f64_from_u52(x), -f64_of(M == kTpF64Tight ? tp_centre<M>(v, p) : v));
         return f64_canon(__dadd_rn(f64_mulmod(d, f64_of(w.w), f64_of(w.ws), p.qd), f64_from_u52(y)), p.qd, p.qi);
     }
     if (M == kTpNear) return csub(near_reduce(shoup_lazy4(x + 6 * p.q - v, w.w, w.ws, p.q) + y, p.d), p.q);
-    return add_mod(shoup_mul(sub_mod(x, tp_canon<M>(v, p, r1), p.q), w.w, w.ws, p.q), y, p.q);
+    return add_mod(shoup_mul(sub_mod(x, tp_canon<M>(v, p), p.q), w.w, w.ws, p.q), y, p.q);
 }
 // v x, canonical; x a canonical residue
 template <int M>
@@ -130,7 +130,7 @@ LB_D u64 tp_end_product(const u64 v, const u64 x, const TpPrime &p, const u64 r0
         return f64_canon(f64_mulmod(f64_of(M == kTpF64Tight ? tp_centre<M>(v, p) : v), w, __dmul_rn(w, p.qi), p.qd), p.qd, p.qi);
     }
     if (M == kTpNear) return csub(near_fold(mul_wide(v, x), p.d), p.q);
-    return barrett128(mul_wide(tp_canon<M>(v, p, r1), x), p.q, r0, r1);
+    return barrett128(mul_wide(tp_canon<M>(v, p), x), p.q, r0, r1);
 }
 
 // S forward stages on canonical or settled values; tw(u, b): twiddle of block b at stage u
@@ -155,10 +155,6 @@ LB_D void tp_fwd(u64 (&v)[1 << S], const TpPrime &p, const TW &tw)
                     if (u == 3) x = near_reduce(x, p.d);
                     const u64 t = shoup_lazy4(y, w.x, w.y, p.q);
                     y = x + (p.q << 2) - t;
-                    x = x + t;
-                } else if (M == kTpLazy) {
-                    const u64 t = shoup_lazy(y, w.x, w.y, p.q);
-                    y = x + (p.q << 1) - t;
                     x = x + t;
                 } else {
                     const u64 q4 = p.q << 2, t = shoup_lazy4(y, w.x, w.y, p.q);

@@ -245,7 +245,6 @@ __global__ void __launch_bounds__(ColShape<A>::THREADS, ColShape<A>::THREADS == 
     case kTpF64: col_fwd_body<A, kTpF64, PLAIN>(sm, fr, mid, tile); break;
     case kTpF64Tight: col_fwd_body<A, kTpF64Tight, PLAIN>(sm, fr, mid, tile); break;
     case kTpNear: col_fwd_body<A, kTpNear, PLAIN>(sm, fr, mid, tile); break;
-    case kTpLazy: col_fwd_body<A, kTpLazy, PLAIN>(sm, fr, mid, tile); break;
     default: col_fwd_body<A, kTpStrict, PLAIN>(sm, fr, mid, tile); break;
     }
 }
@@ -309,10 +308,9 @@ LB_D void row_fwd_body(u64 *srow, const NttK &a, const RowPlace &w, const ModCon
         row_transpose(v, srow, t);
         tg = row_twiddles(tw, logN, w.r, t, true);
     }
-    const u64 r1 = mc->r1;
     if (PLAIN || (!a.aux && !a.mul2)) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = tp_canon<M>(v[k], p, r1);
+        for (int k = 0; k < 16; ++k) v[k] = tp_canon<M>(v[k], p);
     }
     row_transpose(v, srow, t); // back to neighbouring threads on neighbouring coefficients
     if (!PLAIN && a.aux) {
@@ -333,12 +331,12 @@ LB_D void row_fwd_body(u64 *srow, const NttK &a, const RowPlace &w, const ModCon
                 for (int k = 0; k < 4; ++k) y[k] = add[16 * (h + k)];
             }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) v[h + k] = tp_end_scaled<M>(v[h + k], x[k], y[k], scal, p, r1);
+            for (int k = 0; k < 4; ++k) v[h + k] = tp_end_scaled<M>(v[h + k], x[k], y[k], scal, p);
         }
     } else if (!PLAIN && a.mul2) {
         const u64 *mul0 = a.mul2 + ((size_t)w.rr << logN) + base, *mul1 = mul0 + ((size_t)a.per_group << logN);
         u64 *const dst1 = dst + ((size_t)a.per_group << logN);
-        const u64 r0 = mc->r0;
+        const u64 r0 = mc->r0, r1 = mc->r1;
 #pragma unroll
         for (int h = 0; h < 16; h += 4) {
             u64 x[4], y[4];
@@ -379,7 +377,6 @@ __global__ void __launch_bounds__(kRowThreads, 6) ntt_fwd_row_kernel(const __gri
     case kTpF64: row_fwd_body<kTpF64, PLAIN>(srow, a, w, mc, tw); break;
     case kTpF64Tight: row_fwd_body<kTpF64Tight, PLAIN>(srow, a, w, mc, tw); break;
     case kTpNear: row_fwd_body<kTpNear, PLAIN>(srow, a, w, mc, tw); break;
-    case kTpLazy: row_fwd_body<kTpLazy, PLAIN>(srow, a, w, mc, tw); break;
     default: row_fwd_body<kTpStrict, PLAIN>(srow, a, w, mc, tw); break;
     }
 }
