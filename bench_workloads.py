@@ -176,7 +176,7 @@ class KrumWorkload:
         n = ek.N
         per_limb = (n // 2) * (self.log_slots + 1)
         roofs = [ek.lb.butterfly_rate(v) / per_limb * 16 * n / 1e9 for v in (0, 3)]
-        return {"int_strict_60bit": roofs[0], "fp64_40bit": roofs[1], "chain_mean": 2.0 / (1.0 / roofs[0] + 1.0 / roofs[1])}
+        return {"near_60bit": roofs[0], "fp64_40bit": roofs[1], "chain_mean": 2.0 / (1.0 / roofs[0] + 1.0 / roofs[1])}
 
     # -- CPU baseline -----------------------------------------------------------------------------------
     def cpu_sample(self, threads):
@@ -384,7 +384,7 @@ class NttWorkload:
         """arithmetic ceiling of the transform: the register-only butterfly rate converted to transform traffic"""
         per_limb = (self.N // 2) * self.logn
         to_gbs = lambda rate: rate / per_limb * 16 * self.N / 1e9
-        names = ["int_strict", "int_lazy", "fp64_50bit", "fp64_40bit"]
+        names = ["near_60bit", "integer", "fp64_50bit", "fp64_40bit"]
         out = {n: to_gbs(self.ctx.butterfly_rate(i)) for i, n in enumerate(names)}
         out["this_workload"] = to_gbs(self.ctx.butterfly_rate())  # the variant this workload's primes take
         return out

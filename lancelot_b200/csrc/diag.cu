@@ -8,13 +8,13 @@
 
 #include "../../include/lancelot_b200_diag.h"
 #include "context.h"
-#include "ntt_butterfly.cuh"
+#include "ntt_stages.cuh"
 
 namespace lb {
 
-// the transform kernels' launch shape (ntt.cu): the probe runs at their occupancy
-constexpr int kNttThreads = 256;
-constexpr int kNttMinBlocks = 3;
+// the column kernels' launch shape (ntt_twopass.cuh): the probe runs at their occupancy
+constexpr int kProbeThreads = 256;
+constexpr int kProbeBlocks = 3;
 
 static unsigned long long g_launches = 0;
 unsigned long long launch_count() { return g_launches; }
@@ -59,70 +59,54 @@ void count_launch(const char *name, cudaStream_t stream, double bytes)
 }
 
 // ---- arithmetic ceiling probe -------------------------------------------------------------------
-// The same forward butterfly as the transform kernels, on registers only (no shared or global
-// memory traffic inside the loop), at the transform kernels' occupancy.  Its rate is the ceiling
-// the modular arithmetic of that butterfly variant sets for any NTT schedule on this GPU; one
-// limb of N points needs (N/2) log2 N butterflies for 16 N bytes of traffic.
-template <int MODE>
-__global__ void __launch_bounds__(kNttThreads, kNttMinBlocks) butterfly_probe_kernel(u64 *out, const u64 q, const u64 w0, const u64 ws0,
-                                                                                       const int iters)
+// The four forward stages a thread of the two-kernel transforms takes at a time, with the reduction behind them, on registers only
+// but for twiddles from a table that stays in L1, at the column kernels' occupancy.  Its rate is the ceiling the modular arithmetic
+// of a prime class sets for these transforms on this GPU; one limb of N points needs (N/2) log2 N butterflies.
+constexpr int kProbeTwiddles = 16 * 16;
+template <int M>
+__global__ void __launch_bounds__(kProbeThreads, kProbeBlocks) butterfly_probe_kernel(u64 *out, const u64 q, const ulonglong2 *tw,
+                                                                                      const int iters)
 {
-    u64 v[8];
+    const TpPrime p = tp_prime<M>(q);
+    u64 v[16];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = (u64)threadIdx.x * 8 + i + blockIdx.x;
-    if (is_f64_mode(MODE)) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = bits_of(f64_from_u52(v[i]));
-    }
-    const u64 q2 = bf_scalar_q2<MODE>(q), q1 = bf_scalar_q<MODE>(q);
+    for (int i = 0; i < 16; ++i) v[i] = tp_load<M>((u64)threadIdx.x * 16 + i + blockIdx.x);
     for (int it = 0; it < iters; ++it) {
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int half = 4 >> s;
-#pragma unroll
-            for (int b = 0; b < (1 << s); ++b) {
-                // twiddles that differ per thread and stage, so that nothing is hoisted out of the loop
-                const ulonglong2 w = is_f64_mode(MODE) ? make_ulonglong2(bits_of(f64_of(w0) + (double)(threadIdx.x + b)), bits_of(f64_of(ws0) * (double)(1 + s)))
-                                                  : make_ulonglong2(w0 + threadIdx.x + b, ws0 + threadIdx.x + s);
-#pragma unroll
-                for (int i = 0; i < half; ++i) fwd_bf<MODE>(v[b * 2 * half + i], v[b * 2 * half + i + half], w, q1, q2);
-            }
-        }
-        // keep the lazy ranges bounded, as the closing reduction does
-        if (MODE == kIntLazy) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] &= 0x03FFFFFFFFFFFFFFull;
-        }
-        if (is_f64_mode(MODE)) { // one centred reduction per element and radix-8 pass: what the tight variant does
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = bits_of(f64_centre(f64_of(v[i]), f64_of(q1), f64_of(q2)));
-        }
+        const ulonglong2 *t = tw + (it & 15) * 16; // others each time, so that nothing is hoisted out of the loop
+        tp_fwd<4, M>(v, p, [&](const int u, const int b) { return __ldg(t + (1 << u) - 1 + b); });
+        tp_settle<M>(v, p); // nothing for primes below 2^47: the 3000 q their values grow to here stay finite
     }
     u64 acc = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc ^= v[i];
+    for (int i = 0; i < 16; ++i) acc ^= v[i];
     out[(size_t)blockIdx.x * blockDim.x + threadIdx.x] = acc;
 }
 
-// mode: 0 integer strict, 1 integer lazy, 2 all on the FP64 pipe at a 50-bit prime, 3 all on the FP64 pipe at a 40-bit prime,
-// -1 the variant the context's first prime takes.
-int probe_butterfly_rate(Context *ctx, int mode, double *butterflies_per_second)
+// variant: 0 near 2^60, 1 the other integers, 2 all on the FP64 pipe at a 50-bit prime, 3 the same at a 40-bit prime,
+// -1 the one the context's first prime takes.
+int probe_butterfly_rate(Context *ctx, int variant, double *butterflies_per_second)
 {
-    if (mode < 0) {
-        const u64 q0 = ctx->hp.q[0];
-        mode = q0 < kF64PrimeLimit ? kF64 : q0 < kF64TightPrimeLimit ? kF64Tight : (q0 >> 58) == 0 ? kIntLazy : kIntStrict;
-    }
-    if (mode > kF64) {
+    static const int mode_of[4] = {kTpNear, kTpStrict, kTpF64Tight, kTpF64};
+    if (variant > 3) {
         set_error("butterfly variant must be 0..3 or -1");
         return LB_ERR_INVALID_ARG;
     }
-    const int blocks = ctx->sm_count * kNttMinBlocks, iters = 2000;
-    int rc = ctx->ensure_workspace((size_t)blocks * kNttThreads * sizeof(u64));
+    for (int v = 0; variant < 0 && v < 4; ++v)
+        if (mode_of[v] == tp_fwd_mode(ctx->hp.q[0])) variant = v;
+    const int blocks = ctx->sm_count * kProbeBlocks, iters = 1000;
+    int rc = ctx->ensure_workspace(kProbeTwiddles * sizeof(ulonglong2) + (size_t)blocks * kProbeThreads * sizeof(u64));
     if (rc) return rc;
-    u64 *out = reinterpret_cast<u64 *>(ctx->ws);
+    ulonglong2 *tw = reinterpret_cast<ulonglong2 *>(ctx->ws);
+    u64 *out = reinterpret_cast<u64 *>(tw + kProbeTwiddles);
     // any odd modulus of the variant's size gives the variant's instruction stream
-    static const u64 size_of_mode[4] = {(u64(1) << 60) - 93, (u64(1) << 57) - 13, (u64(1) << 50) - 27, (u64(1) << 40) - 87};
-    const u64 q = size_of_mode[mode], w = h_twiddle_value(q / 3, q), ws = h_twiddle_quot(q / 3, q);
+    static const u64 modulus_of[4] = {(u64(1) << 60) - 93, (u64(1) << 57) - 13, (u64(1) << 50) - 27, (u64(1) << 40) - 87};
+    const u64 q = modulus_of[variant];
+    ulonglong2 table[kProbeTwiddles];
+    for (int i = 0; i < kProbeTwiddles; ++i) {
+        const u64 w = (u64(0x9E3779B97F4A7C15) * (i + 1)) % q;
+        table[i] = make_ulonglong2(h_twiddle_value(w, q), h_twiddle_quot(w, q));
+    }
+    LB_CUDA(cudaMemcpy(tw, table, sizeof(table), cudaMemcpyHostToDevice));
     cudaEvent_t e0, e1;
     LB_CUDA(cudaEventCreate(&e0));
     LB_CUDA(cudaEventCreate(&e1));
@@ -130,12 +114,13 @@ int probe_butterfly_rate(Context *ctx, int mode, double *butterflies_per_second)
     for (int rep = 0; rep < 4; ++rep) {
         LB_CUDA(cudaEventRecord(e0, 0));
         count_launch("butterfly_probe_kernel", nullptr);
-        switch (mode) {
-        case kIntStrict: butterfly_probe_kernel<kIntStrict><<<blocks, kNttThreads>>>(out, q, w, ws, iters); break;
-        case kIntLazy: butterfly_probe_kernel<kIntLazy><<<blocks, kNttThreads>>>(out, q, w, ws, iters); break;
-        case kF64Tight: butterfly_probe_kernel<kF64Tight><<<blocks, kNttThreads>>>(out, q, w, ws, iters); break;
-        default: butterfly_probe_kernel<kF64><<<blocks, kNttThreads>>>(out, q, w, ws, iters); break;
+        switch (mode_of[variant]) {
+        case kTpNear: butterfly_probe_kernel<kTpNear><<<blocks, kProbeThreads>>>(out, q, tw, iters); break;
+        case kTpStrict: butterfly_probe_kernel<kTpStrict><<<blocks, kProbeThreads>>>(out, q, tw, iters); break;
+        case kTpF64Tight: butterfly_probe_kernel<kTpF64Tight><<<blocks, kProbeThreads>>>(out, q, tw, iters); break;
+        default: butterfly_probe_kernel<kTpF64><<<blocks, kProbeThreads>>>(out, q, tw, iters); break;
         }
+        LB_CUDA(cudaGetLastError());
         LB_CUDA(cudaEventRecord(e1, 0));
         LB_CUDA(cudaEventSynchronize(e1));
         float ms = 0;
@@ -144,10 +129,9 @@ int probe_butterfly_rate(Context *ctx, int mode, double *butterflies_per_second)
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    *butterflies_per_second = (double)blocks * kNttThreads * iters * 12.0 / (best * 1e-3);
+    *butterflies_per_second = (double)blocks * kProbeThreads * iters * 32.0 / (best * 1e-3);
     return LB_OK;
 }
-
 
 } // namespace lb
 
