@@ -708,9 +708,14 @@ static const char *kernel_label(bool forward, const NttK &k)
     return !forward ? "ntt_inv_kernel" : plain_input(k) ? "ntt_fwd_kernel(plain input)" : "ntt_fwd_kernel(fused input)";
 }
 
+// algorithmic bytes of a transform for the diagnostics: what its source, its limb rows (once) and its fused ends hold
+struct NttBytes {
+    double in, rows, ends;
+};
+
 // rings below 4096 points (LOGC == 0) and of 131072 points (LOGC == 4)
 template <int LOGC>
-static int launch(bool forward, const NttK &k, int rows, size_t smem, cudaStream_t stream, double bytes)
+static int launch(bool forward, const NttK &k, int rows, size_t smem, cudaStream_t stream, const NttBytes &b)
 {
     auto kern = forward ? ntt_fwd_kernel<LOGC> : ntt_inv_kernel<LOGC>;
     // function attributes belong to the device the kernel image is loaded on
@@ -736,7 +741,7 @@ static int launch(bool forward, const NttK &k, int rows, size_t smem, cudaStream
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    count_launch(kernel_label(forward, k), stream, bytes);
+    count_launch(kernel_label(forward, k), stream, b.in + b.rows + b.ends);
     LB_CUDA(cudaLaunchKernelEx(&cfg, kern, k));
     return LB_OK;
 }
@@ -769,7 +774,7 @@ static void share_rows(NttK &k, int n_groups)
 }
 
 template <int A>
-static int launch_twopass(bool forward, NttK &k, int rows, cudaStream_t stream, double bytes)
+static int launch_twopass(bool forward, NttK &k, int rows, cudaStream_t stream, const NttBytes &b)
 {
     using C = ColShape<A>;
     share_rows(k, rows / k.per_group);
@@ -777,14 +782,15 @@ static int launch_twopass(bool forward, NttK &k, int rows, cudaStream_t stream, 
     const long row_grid = (long)((k.n_polys + (1 << k.log_polys) - 1) >> k.log_polys) * k.poly_step * k.per_group << (A - 3 + k.log_polys);
     const bool plain = plain_input(k);
     int rc;
-    count_launch(kernel_label(forward, k), stream, bytes);
     if (forward) {
+        count_launch(plain ? "ntt_fwd_col_kernel(plain)" : "ntt_fwd_col_kernel(fused)", stream, b.in + b.rows);
         if ((rc = launch_serial(plain ? ntt_fwd_col_kernel<A, true> : ntt_fwd_col_kernel<A, false>, k, col_grid, C::THREADS, stream))) return rc;
-        count_launch(kernel_label(forward, k), stream);
+        count_launch(plain ? "ntt_fwd_row_kernel(plain)" : "ntt_fwd_row_kernel(fused)", stream, 2 * b.rows + b.ends);
         return launch_serial(plain ? ntt_fwd_row_kernel<true> : ntt_fwd_row_kernel<false>, k, row_grid, kRowThreads, stream);
     }
+    count_launch("ntt_inv_row_kernel", stream, b.in + b.rows);
     if ((rc = launch_serial(ntt_inv_row_kernel, k, row_grid, kRowThreads, stream))) return rc;
-    count_launch(kernel_label(forward, k), stream);
+    count_launch("ntt_inv_col_kernel", stream, 2 * b.rows);
     return launch_serial(ntt_inv_col_kernel<A>, k, col_grid, C::THREADS, stream);
 }
 
@@ -847,31 +853,31 @@ static int run(Context *ctx, const NttJob &job, bool forward, cudaStream_t strea
     for (int i = 0; i < pl.npass; ++i) k.S[i] = pl.S[i];
     const size_t n_loc = size_t(1) << logn_loc;
     const size_t smem = (n_loc + (n_loc >> 4) + 2) * sizeof(u64);
-    // algorithmic bytes of this launch (diagnostics): rows written once; plain rows read once; fused loaders read the
-    // group's source rows once per group, plus the rows the epilogue and the prologue fold in
+    // diagnostics: rows written once; plain rows read once; fused loaders read the group's source rows once per group, plus the
+    // rows the prologue and the epilogue fold in
     const double limb = 8.0 * (double)hp.N;
     const int live = job.per_group - (job.skip_hi > job.skip_lo ? job.skip_hi - job.skip_lo : 0);
     const double out_rows = (double)job.n_groups * live;
-    double bytes = out_rows * limb;
-    if (job.digit_alpha > 0) bytes += (double)job.n_groups * job.digit_alpha * limb;
-    else if (job.bconv_n > 0) bytes += (double)job.n_groups * job.bconv_n * limb;
-    else if (job.small) bytes += (double)job.n_groups * (double)hp.N; // one byte per coefficient and group
-    else bytes += out_rows * limb;
+    NttBytes b = {0, out_rows * limb, 0};
+    if (job.digit_alpha > 0) b.in = (double)job.n_groups * job.digit_alpha * limb;
+    else if (job.bconv_n > 0) b.in = (double)job.n_groups * job.bconv_n * limb;
+    else if (job.small) b.in = (double)job.n_groups * (double)hp.N; // one byte per coefficient and group
+    else b.in = out_rows * limb;
     const double outer = (double)job.n_groups / k.split;
-    if (job.aux) bytes += out_rows * limb;
-    if (job.add) bytes += outer * (job.add_inner < k.split ? job.add_inner : k.split) * live * limb;
-    if (job.add1) bytes += outer * live * limb;
-    if (job.presub) bytes += outer * (k.presub_inner < k.split ? k.presub_inner : k.split) * live * limb;
-    if (job.esmall) bytes += outer * (double)hp.N;
-    if (job.mul2) bytes += out_rows * limb + 2.0 * job.per_group * limb; // a second output row per row, the two fixed rows once
+    if (job.aux) b.ends += out_rows * limb;
+    if (job.add) b.ends += outer * (job.add_inner < k.split ? job.add_inner : k.split) * live * limb;
+    if (job.add1) b.ends += outer * live * limb;
+    if (job.presub) b.in += outer * (k.presub_inner < k.split ? k.presub_inner : k.split) * live * limb;
+    if (job.esmall) b.in += outer * (double)hp.N;
+    if (job.mul2) b.ends += out_rows * limb + 2.0 * job.per_group * limb; // a second output row per row, the two fixed rows once
     switch (hp.logN) {
-    case 12: return launch_twopass<4>(forward, k, rows, stream, bytes);
-    case 13: return launch_twopass<5>(forward, k, rows, stream, bytes);
-    case 14: return launch_twopass<6>(forward, k, rows, stream, bytes);
-    case 15: return launch_twopass<7>(forward, k, rows, stream, bytes);
-    case 16: return launch_twopass<8>(forward, k, rows, stream, bytes);
-    case 17: return launch<4>(forward, k, rows, smem, stream, bytes);
-    default: return launch<0>(forward, k, rows, smem, stream, bytes);
+    case 12: return launch_twopass<4>(forward, k, rows, stream, b);
+    case 13: return launch_twopass<5>(forward, k, rows, stream, b);
+    case 14: return launch_twopass<6>(forward, k, rows, stream, b);
+    case 15: return launch_twopass<7>(forward, k, rows, stream, b);
+    case 16: return launch_twopass<8>(forward, k, rows, stream, b);
+    case 17: return launch<4>(forward, k, rows, smem, stream, b);
+    default: return launch<0>(forward, k, rows, smem, stream, b);
     }
 }
 

@@ -878,7 +878,7 @@ struct MaskArgs {
 // outer two at the end of a window (words below 2^61, so 32 products stay below 2^127).  Four clients unrolled and six blocks per
 // SM keep enough loads in flight; four chunks per thread lost to the registers of their 128-bit sums, and so did the prime's
 // constants held in registers (264 bytes spilt; they are read where the sums are reduced).  20 clients x 16 chunks of N = 2^16
-// 307.9 -> 206.3 us (4.8 TB/s), 3 clients x 3 chunks 16.5 -> 14.4; a second, idle chunk in place of the odd one took 20.5.
+// 307.9 -> 206.3 us (5.2 TB/s), 3 clients x 3 chunks 16.5 -> 14.4; a second, idle chunk in place of the odd one took 20.5.
 constexpr int kMaskChunks = 2;
 
 // C chunks from chunk c0 on, one coefficient of each
