@@ -241,10 +241,12 @@ __global__ void __launch_bounds__(ColShape<A>::THREADS, ColShape<A>::THREADS == 
     FwdRow fr;
     if (!fwd_row_setup(a, row, fr)) return;
     u64 *mid = a.mid ? a.mid + ((size_t)row << a.logN) : fr.dst;
+    // the order of the classes is the order of their code, here and in the row kernel: with the FP64 classes first, 768 limbs of
+    // 50 bits took 379.8 us instead of 362.9 and the 10-client round at N = 2^15 14.20 ms instead of 14.02
     switch (tp_fwd_mode(fr.q)) {
-    case kTpF64: col_fwd_body<A, kTpF64, PLAIN>(sm, fr, mid, tile); break;
-    case kTpF64Tight: col_fwd_body<A, kTpF64Tight, PLAIN>(sm, fr, mid, tile); break;
     case kTpNear: col_fwd_body<A, kTpNear, PLAIN>(sm, fr, mid, tile); break;
+    case kTpF64Tight: col_fwd_body<A, kTpF64Tight, PLAIN>(sm, fr, mid, tile); break;
+    case kTpF64: col_fwd_body<A, kTpF64, PLAIN>(sm, fr, mid, tile); break;
     default: col_fwd_body<A, kTpStrict, PLAIN>(sm, fr, mid, tile); break;
     }
 }
@@ -374,9 +376,9 @@ __global__ void __launch_bounds__(kRowThreads, 6) ntt_fwd_row_kernel(const __gri
     const ulonglong2 *tw = a.tw + ((size_t)tbl << a.logN);
     u64 *srow = sm + (threadIdx.x >> 4) * kRowPad;
     switch (tp_fwd_mode(mc->q)) {
-    case kTpF64: row_fwd_body<kTpF64, PLAIN>(srow, a, w, mc, tw); break;
-    case kTpF64Tight: row_fwd_body<kTpF64Tight, PLAIN>(srow, a, w, mc, tw); break;
     case kTpNear: row_fwd_body<kTpNear, PLAIN>(srow, a, w, mc, tw); break;
+    case kTpF64Tight: row_fwd_body<kTpF64Tight, PLAIN>(srow, a, w, mc, tw); break;
+    case kTpF64: row_fwd_body<kTpF64, PLAIN>(srow, a, w, mc, tw); break;
     default: row_fwd_body<kTpStrict, PLAIN>(srow, a, w, mc, tw); break;
     }
 }
