@@ -1,8 +1,8 @@
 """Bit-exact parity of the CUDA path against the CPU oracle at the sizes the benchmarks run:
 N = 2^15 and 2^16 with Lancelot's chain {60,40,40 | 60}, and N = 2^16 with 24 data primes and eight
-special primes (alpha = 8, dnum = 3).  These ring degrees take other code paths than the small cases
-(clusters of 4 and 8 CTAs per limb, the fixed-schedule transforms and their fused loaders), so the
-small-ring digests do not cover them.  Needs a B200; run with -m gpu."""
+special primes (alpha = 8, dnum = 3).  These ring degrees take other shapes of the column kernels than the
+small cases (128 and 256 rows, two groups of stages per column), and their fused loaders, so the small-ring
+digests do not cover them.  Needs a B200; run with -m gpu."""
 import numpy as np
 import pytest
 
