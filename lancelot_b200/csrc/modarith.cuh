@@ -1,9 +1,8 @@
 // 64-bit modular arithmetic shared by host precompute and device kernels.
 //
-// Device code keeps residues lazily reduced inside a kernel (forward butterflies in
-// [0,4q), inverse in [0,2q)) and always stores the canonical residue in [0,q), which is
-// what every stage of the reference library leaves in memory
-// (cahel-main/src/ntt/fntt_2d.cu:860-866, cahel-main/include/uintmodmath.cuh:112-259).
+// Device code keeps residues lazily reduced inside an operation (the ranges are stated at the butterflies), between the two
+// kernels of a transform also in memory, and leaves the canonical residue in [0,q) when the operation is done, as every stage of
+// the reference library does (cahel-main/src/ntt/fntt_2d.cu:860-866, cahel-main/include/uintmodmath.cuh:112-259).
 #pragma once
 #include <cstdint>
 #include <type_traits>
@@ -69,8 +68,8 @@ inline u64 h_shoup(u64 w, u64 q) { return (u64)(((u128)w << 64) / q); }
 // Primes below 2^50: the whole butterfly runs on the FP64 pipe.  Residues travel through the
 // transform as integer-valued doubles (their bit patterns sit in the same 64-bit words), products
 // are formed error-free with fused multiply-adds.  Below 2^47 values may grow over all forward stages
-// without a reduction (13 q < 2^51); from 2^47 up they are centred once per pass (ntt_butterfly.cuh).
-// Their twiddle entries are (double(w), double(w / q)).
+// without a reduction (13.5 q < 2^51); from 2^47 up they are centred every three or four stages.
+// Their twiddle entries are (double(w), double(w / q)) with w the representative in (-q/2, q/2).
 constexpr u64 kF64TightPrimeLimit = u64(1) << 50; // below it the butterflies run on the FP64 pipe: 2q stays below 2^51
 constexpr u64 kF64PrimeLimit = u64(1) << 47;
 
@@ -130,12 +129,13 @@ LB_D double f64_from_u52(u64 x) { return __dadd_rn(__longlong_as_double((long lo
 // back: a double holding an integer of [0, 2^52)
 LB_D u64 u52_from_f64(double d) { return (u64)__double_as_longlong(__dadd_rn(d, 4503599627370496.0)) & 0x000FFFFFFFFFFFFFull; }
 
-// r = y w - Q q with Q the integer nearest to y w / q: r is congruent to y w and |r| <= 0.75 q.
-// Needs integer-valued |y| < 2^51, w < q < 2^47, wq = double(w / q).  y w is split error-free into
-// h + l (l = fma(y, w, -h) is exact); Q comes from one fused multiply-add into 1.5 * 2^52, whose
-// rounding is the rounding to an integer (|y wq| < 2^51 keeps the sum inside [2^52, 2^53)); the
-// estimate is off by at most 0.5 + 2^-2.  h - Q q = (y w - Q q) - l is an integer below 2^50 in
-// magnitude, so the second fused multiply-add is exact, and so is the final sum.
+// r = y w - Q q with Q an integer next to y w / q: r is congruent to y w and |r| <= 0.75 q.
+// Needs integer-valued |y| <= 2^52, |w| <= q < 2^50, |y w / q| <= 2^51 and wq = w / q rounded once; rounded
+// twice (w times the rounded 1 / q) the remainder is bounded by q.  y w is split error-free into h + l
+// (l = fma(y, w, -h) is exact); Q comes from one fused multiply-add into 1.5 * 2^52, whose rounding is the
+// rounding to an integer (the sum stays inside [2^52, 2^53)); the estimate is off by at most 0.5 and the
+// error of wq, 2^51 * 2^-53.  h - Q q = r - l with |l| <= 2^48 (half a unit of |y w| <= 2^101) is an integer
+// below 2^52 in magnitude, so the second fused multiply-add is exact, and so is the final sum.
 LB_D double f64_mulmod(const double y, const double w, const double wq, const double q)
 {
     const double h = __dmul_rn(y, w);
@@ -168,9 +168,10 @@ LB_D u64 shoup_lazy(u64 x, u64 w, u64 ws, u64 q)
 // than one), so the result is congruent to x w and lies in [0, 4q).  For the butterflies, which only need a bound.
 // Spelled out in 32-bit steps: the quotient's cross terms join the high product on a carry chain and both low products go
 // into one accumulator (with -q, so that both only add, and a multiply-add takes its addend for free): nine multiplier and
-// four adder instructions, 39.6 instead of 42.8 cycles per butterfly and SM partition in a register-only loop against the
-// same steps written on 64-bit words, which the compiler pads with moves.  B200 issues a 32 x 32 + 32 multiplication at 64
-// lanes per clock and SM and one whose high half is used at 32, so the quotient is two thirds of the cost.
+// four adder instructions.  Against the same steps on 64-bit words (shoup_lazy4_words below), which the compiler pads with
+// moves: 37.9 instead of 42.9 cycles per butterfly and SM partition in the four stages of a prime near 2^60 on registers only,
+// 768 limbs of N = 2^16 near 2^60 542 instead of 590 us forward and 598 instead of 636 inverse.  B200 issues a 32 x 32 + 32
+// multiplication at 64 lanes per clock and SM and one whose high half is used at 32, so the quotient is two thirds of the cost.
 LB_D u64 shoup_lazy4(u64 x, u64 w, u64 ws, u64 q)
 {
     u64 r;
@@ -308,8 +309,8 @@ LB_D u64 f64_fold64(const u64 x, const ModConst &m)
 }
 // a signed integer of magnitude below 2^51 (two's complement) as a double
 LB_D double f64_from_s52(const u64 x) { return __dadd_rn(f64_of(x + 0x4338000000000000ull), -6755399441055744.0); }
-// (hi:lo) mod q as an integer-valued double of magnitude at most 1.3 q, for 2^34 <= q < 2^50 and hi < 2^52:
-// |hi c64 / q| <= 2^51 is the range of the quotient in f64_mulmod
+// (hi:lo) mod q as an integer-valued double of magnitude at most 1.5 q (0.75 q from the high half, q / 2 + 2^32 from the low one),
+// for 2^34 <= q < 2^50 and hi < 2^52: |hi c64 / q| <= 2^51 is the range of the quotient in f64_mulmod
 LB_D double f64_fold(const u128d z, const ModConst &m)
 {
     const double h = f64_mulmod(f64_from_u52(z.hi), m.c64, m.c64q, m.qd);

@@ -1,5 +1,4 @@
-// The modular butterflies of the transform kernels (ntt.cu), shared with the register-only
-// rate probe of the diagnostics (diag.cu).
+// The modular butterflies of the one-kernel transforms (ntt.cu); those of the two-kernel ones are in ntt_stages.cuh.
 #pragma once
 #include "modarith.cuh"
 
