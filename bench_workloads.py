@@ -19,9 +19,9 @@ WIDE_BITS = [60] + [50] * 23 + [60] * 8
 # bytes of that same launch; the summary each pair comes from is named.  bench.py scales a kernel's algorithmic
 # bytes by this ratio for "traffic"; a kernel without a capture reports null.
 NCU_TRAFFIC = {
-    # mod-down transform of 128 encryptions, N = 2^16: 750.1 MB read + 386.7 MB written
-    "ntt_fwd_kernel(fused input)": {"dram_bytes": 1136815360, "algorithmic_bytes": 1149239296,
-                                    "summary": "profiles/ntt_fwd_fused_encrypt_batch128.md"},
+    # mod-down transform of 128 encryptions, N = 2^16: 344.3 MB read + 363.9 MB written by its column kernel, 817.5 + 375.2 by the rows
+    "ntt_fwd_col_kernel(fused)": {"dram_bytes": 708212480, "algorithmic_bytes": 746586112, "summary": "profiles/ntt_two_kernel_n65536.md"},
+    "ntt_fwd_row_kernel(fused)": {"dram_bytes": 1192704768, "algorithmic_bytes": 1207959552, "summary": "profiles/ntt_two_kernel_n65536.md"},
     # <2,2> tile of the 10-client round, N = 2^15: 641.8 MB read + 11.9 MB written
     "krum_tile_kernel": {"dram_bytes": 653734400, "algorithmic_bytes": 651165696, "summary": "profiles/krum_tile_kernel_c4.md"},
 }

@@ -783,7 +783,9 @@ static int launch_twopass(bool forward, NttK &k, int rows, cudaStream_t stream, 
     const bool plain = plain_input(k);
     int rc;
     if (forward) {
-        count_launch(plain ? "ntt_fwd_col_kernel(plain)" : "ntt_fwd_col_kernel(fused)", stream, b.in + b.rows);
+        // a conversion of several rows reads them again for every target: its own label, so that no other launch's traffic stands for it
+        count_launch(plain ? "ntt_fwd_col_kernel(plain)" : k.bconv_mat ? "ntt_fwd_col_kernel(conversion)" : "ntt_fwd_col_kernel(fused)", stream,
+                     b.in + b.rows);
         if ((rc = launch_serial(plain ? ntt_fwd_col_kernel<A, true> : ntt_fwd_col_kernel<A, false>, k, col_grid, C::THREADS, stream))) return rc;
         count_launch(plain ? "ntt_fwd_row_kernel(plain)" : "ntt_fwd_row_kernel(fused)", stream, 2 * b.rows + b.ends);
         return launch_serial(plain ? ntt_fwd_row_kernel<true> : ntt_fwd_row_kernel<false>, k, row_grid, kRowThreads, stream);
